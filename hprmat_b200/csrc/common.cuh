@@ -87,6 +87,9 @@ template <> struct PivotKey<float2> {
   __device__ static __forceinline__ int row(unsigned long long k) {
     return (int)(0xFFFFFFFFu - (unsigned)(k & 0xFFFFFFFFull));
   }
+  // the key of value v in row `row` as (low, high) words, and the row of such a pair
+  __device__ static __forceinline__ uint2 key2(float2 v, int row) { return make_uint2(~(unsigned)row, mag(v)); }
+  __device__ static __forceinline__ int row2(uint2 k) { return (int)~k.x; }
 };
 template <> struct PivotKey<double2> {
   using M = unsigned long long;
@@ -98,6 +101,11 @@ template <> struct PivotKey<double2> {
     return (m << 20) | (unsigned long long)(0xFFFFFu - (unsigned)row);
   }
   __device__ static __forceinline__ int row(unsigned long long k) { return (int)(0xFFFFFu - (unsigned)(k & 0xFFFFFull)); }
+  __device__ static __forceinline__ uint2 key2(double2 v, int row) {
+    const unsigned long long k = key(mag(v), row);
+    return make_uint2((unsigned)k, (unsigned)(k >> 32));
+  }
+  __device__ static __forceinline__ int row2(uint2 k) { return (int)(0xFFFFFu - (k.x & 0xFFFFFu)); }
 };
 
 // 32-bit key of a non-negative magnitude over the whole double range: the high word of its

@@ -4,7 +4,8 @@
 //
 // Storage: the matrix W is column-major with leading dimension ld (complex elements).
 // Block step s factors columns [k0, k0+ncols) with k0 = s*nb:
-//   1. panel_kernel      -- cooperative launch, the panel rows spread over all SMs and held
+//   1. the panel: panel_reg_kernel (panel.cuh) where the rows fit in one thread-block cluster,
+//      else panel_kernel -- cooperative launch, the panel rows spread over all SMs and held
 //                           in shared memory; one grid barrier per column: every CTA posts
 //                           its local |re|+|im| maximum (the modulus LAPACK's izamax uses)
 //                           and that row, then all CTAs pick the same pivot, swap and
@@ -19,8 +20,6 @@
 // forward solve applies each step's interchanges to the right-hand side just before that
 // step's block column, which is consistent with the factors stored that way.
 #pragma once
-#include <cooperative_groups.h>
-
 #include "common.cuh"
 
 namespace hprmat {
@@ -63,8 +62,7 @@ constexpr int kPanelTraceW = 5 + 160;
 // that orders over the element type's whole range (FP64 panels: magnitudes far outside the
 // float range too), with the lowest row winning among equal moduli.
 
-// End of a panel factorisation, shared by both panel kernels: the CTA's factored rows back
-// into W, its L21 rows into the LU planes (mixed path), and from CTA 0 the pivots, the growth
+// End of a panel factorisation: the CTA's factored rows back into W, its L21 rows into the LU planes (mixed path), and from CTA 0 the pivots, the growth
 // and the step's row-interchange list.
 template <typename T, int NB, int NT>
 __device__ void panel_finish(const PanelArgs<T>& a, const T* P, int rpcp, int r0, int nloc, const int* s_loc_ipiv,
@@ -333,205 +331,11 @@ __global__ void __launch_bounds__(NT, 1) panel_kernel(PanelArgs<T> a) {
 }
 
 // -------------------------------------------------------------------------------------
-// The panel factorisation of panel_kernel for panels whose rows fit in one thread-block
-// cluster (G <= 16 CTAs, the whole grid): the same algorithm and look-ahead, with the
-// per-column exchange in distributed shared memory instead of global memory.  Each CTA pushes
-// its pivot key into every CTA's shared memory and posts its candidate row and (the owner)
-// row j in its own; after the hardware cluster barrier every CTA reduces the G keys locally,
-// picks the same pivot and reads the two rows from their owners (one remote round trip).
-// Double buffering by column parity is safe because a CTA posts column j + 2 only after the
-// barrier of column j + 1, which every CTA reaches after reading column j.  There is no
-// polling: the waits are the cluster barrier's.  Dynamic shared memory: P [NB][rpc|1],
-// urow [NB], candidate rows [2][NB], rows j [2][NB], keys [2][16].
-namespace cgx = cooperative_groups;
-
+// Hardware barrier of a thread-block cluster, for panels that fit in one (panel.cuh).
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 constexpr int kMaxClusterCTAs = 16;
-
-template <typename T>
-__host__ __device__ constexpr size_t panel_cluster_smem(int rpc, int nb) {
-  return ((size_t)nb * (size_t)(rpc | 1) + 5 * (size_t)nb) * sizeof(T) +
-         2 * kMaxClusterCTAs * sizeof(unsigned long long) + 16;
-}
-
-template <typename T, int NB, int NT>
-__global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(PanelArgs<T> a) {
-  using R = typename RealOf<T>::R;
-  cgx::cluster_group cluster = cgx::this_cluster();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int m = a.N - a.k0;
-  const int b = (int)cluster.block_rank();
-  const int r0 = b * a.rpc;
-  const int r1 = min(r0 + a.rpc, m);
-  const int nloc = max(r1 - r0, 0);
-  const int rpcp = a.rpc | 1;
-  T* P = reinterpret_cast<T*>(smem_raw);  // [NB][rpcp] column-major
-  T* urow = P + (size_t)NB * rpcp;        // [NB]
-  T* xrow = urow + NB;                    // [2][NB] candidate row posted by this CTA
-  T* xrowj = xrow + 2 * NB;               // [2][NB] row j, posted by its owner
-  // [2][kMaxClusterCTAs]: every CTA's pivot key, pushed into every CTA before the barrier
-  unsigned long long* xkey = reinterpret_cast<unsigned long long*>(xrowj + 2 * NB);
-  using PK = PivotKey<T>;
-  using PM = typename PK::M;
-  __shared__ PM red_v[NT / 32];
-  __shared__ int red_i[NT / 32];
-  __shared__ int s_piv, s_loc_ipiv[NB];
-  __shared__ unsigned s_growth;
-  const int tid = threadIdx.x;
-  const int ncols = a.ncols;
-
-  for (int c = 0; c < ncols; ++c)
-    for (int lr = tid; lr < nloc; lr += NT)
-      P[(size_t)c * rpcp + lr] = a.W[(size_t)(a.k0 + r0 + lr) + (size_t)(a.k0 + c) * a.ld];
-  if (tid == 0) s_growth = 0u;
-  __syncthreads();
-
-  // column jc's local candidate into s_piv, and its key into slot b of xkey[jc & 1] of every
-  // CTA of the cluster (lane t of warp 0 stores into CTA t)
-  auto candidate = [&](int jc, PM bv, int bi) {
-    for (int o = 16; o > 0; o >>= 1) {
-      PM ov = __shfl_down_sync(0xffffffffu, bv, o);
-      int oi = __shfl_down_sync(0xffffffffu, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-    if ((tid & 31) == 0) { red_v[tid >> 5] = bv; red_i[tid >> 5] = bi; }
-    __syncthreads();
-    if (tid < 32) {
-      bv = (tid < NT / 32) ? red_v[tid] : PM(0);
-      bi = (tid < NT / 32) ? red_i[tid] : 0x7fffffff;
-      for (int o = 16; o > 0; o >>= 1) {
-        PM ov = __shfl_down_sync(0xffffffffu, bv, o);
-        int oi = __shfl_down_sync(0xffffffffu, bi, o);
-        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-      }
-      if (tid == 0) s_piv = bi;
-      const unsigned long long key = __shfl_sync(0xffffffffu, bi != 0x7fffffff ? PK::key(bv, bi) : 0ull, 0);
-      if (tid < a.G) *cluster.map_shared_rank(xkey + (jc & 1) * kMaxClusterCTAs + b, (unsigned)tid) = key;
-    }
-    __syncthreads();
-  };
-  auto post = [&](int jc, bool pend) {
-    const int pb = jc & 1;
-    const int ci = s_piv;
-    const bool have = ci != 0x7fffffff;
-    const bool own = jc >= r0 && jc < r1;
-    for (int c = tid; c < ncols; c += NT) {
-      if (have) {
-        T v = P[(size_t)c * rpcp + (ci - r0)];
-        if (pend && c > jc) cfms(v, P[(size_t)(jc - 1) * rpcp + (ci - r0)], urow[c]);
-        xrow[pb * NB + c] = v;
-      }
-      if (own) {
-        T v = P[(size_t)c * rpcp + (jc - r0)];
-        if (pend && c > jc) cfms(v, P[(size_t)(jc - 1) * rpcp + (jc - r0)], urow[c]);
-        xrowj[pb * NB + c] = v;
-      }
-    }
-  };
-
-  {
-    PM bv = 0;
-    int bi = 0x7fffffff;
-    for (int lr = tid; lr < nloc; lr += NT) {
-      const PM v = PK::mag(P[lr]);
-      if (v > bv) { bv = v; bi = r0 + lr; }
-    }
-    candidate(0, bv, bi);
-    post(0, false);
-    cluster_arrive();
-  }
-  const int warp = tid >> 5, lane = tid & 31;
-  for (int j = 0; j < ncols; ++j) {
-    const int buf = j & 1;
-    cluster_wait();
-    // the largest key names the pivot row (the lowest row among equal moduli); every warp
-    // reduces the G keys, now in local shared memory, itself
-    unsigned long long kmax;
-    {
-      const int lane_ = tid & 31;
-      unsigned long long k = lane_ < a.G ? xkey[buf * kMaxClusterCTAs + lane_] : 0ull;
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long v = __shfl_xor_sync(0xffffffffu, k, o);
-        k = v > k ? v : k;
-      }
-      kmax = k;
-    }
-    const int p = PK::row(kmax);
-    const T* wrow = cluster.map_shared_rank(xrow + buf * NB, (unsigned)(p / a.rpc));
-    const T* jrow = cluster.map_shared_rank(xrowj + buf * NB, (unsigned)(j / a.rpc));
-    unsigned g = 0u;
-    for (int c = tid; c < ncols; c += NT) {
-      T u = wrow[c];
-      urow[c] = u;
-      if (p != j && p >= r0 && p < r1) P[(size_t)c * rpcp + (p - r0)] = jrow[c];
-      if (p != j && j >= r0 && j < r1) P[(size_t)c * rpcp + (j - r0)] = u;
-      if (c >= j) g = max(g, mag_hi((double)cabs1(u)));
-    }
-    if (tid < ((ncols + 31) & ~31)) {
-      for (int o = 16; o > 0; o >>= 1) g = max(g, __shfl_down_sync(0xffffffffu, g, o));
-      if ((tid & 31) == 0 && g > 0u) atomicMax(&s_growth, g);
-    }
-    if (tid == 0) s_loc_ipiv[j] = p;
-    __syncthreads();
-    const T piv = urow[j];
-    const bool zero = (piv.x == R(0) && piv.y == R(0));
-    if (zero && b == 0 && tid == 0) atomicCAS(a.status + SW_INFO, 0, a.k0 + j + 1);
-    const T inv = zero ? czero<T>() : crecip(piv);
-    const int lo = max(j + 1 - r0, 0);
-    if (j + 1 < ncols) {
-      const int jn = j + 1;
-      PM bv = 0;
-      int bi = 0x7fffffff;
-      for (int lr = lo + tid; lr < nloc; lr += NT) {
-        T l = P[(size_t)j * rpcp + lr];
-        if (!zero) {
-          l = cmul(l, inv);
-          P[(size_t)j * rpcp + lr] = l;
-        }
-        T v = P[(size_t)jn * rpcp + lr];
-        cfms(v, l, urow[jn]);
-        P[(size_t)jn * rpcp + lr] = v;
-        const PM av = PK::mag(v);
-        if (av > bv) { bv = av; bi = r0 + lr; }
-      }
-      candidate(jn, bv, bi);
-      post(jn, true);
-      cluster_arrive();
-      constexpr int NW = NT / 32;
-      for (int lr = lo + lane; lr < nloc; lr += 32) {
-        const T l = P[(size_t)j * rpcp + lr];
-        int c = jn + 1 + warp;
-        for (; c + 3 * NW < ncols; c += 4 * NW) {
-          T v[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) v[q] = P[(size_t)(c + q * NW) * rpcp + lr];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            cfms(v[q], l, urow[c + q * NW]);
-            P[(size_t)(c + q * NW) * rpcp + lr] = v[q];
-          }
-        }
-        for (; c < ncols; c += NW) {
-          T v = P[(size_t)c * rpcp + lr];
-          cfms(v, l, urow[c]);
-          P[(size_t)c * rpcp + lr] = v;
-        }
-      }
-      __syncthreads();
-    } else {
-      for (int lr = lo + tid; lr < nloc; lr += NT) {
-        if (!zero) P[(size_t)j * rpcp + lr] = cmul(P[(size_t)j * rpcp + lr], inv);
-      }
-      __syncthreads();
-    }
-  }
-  // no CTA leaves while another may still read its shared memory
-  cluster_arrive();
-  cluster_wait();
-  panel_finish<T, NB, NT>(a, P, rpcp, r0, nloc, s_loc_ipiv, s_growth, b, tid);
-}
 
 // -------------------------------------------------------------------------------------
 // Apply the step's row interchanges to columns [c_begin, c_end) of X and solve with the

@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "coulomb.cuh"
 #include "lu.cuh"
+#include "panel.cuh"
 #include "adjoint.cuh"
 #include "hessenberg.cuh"
 #include "rmat_kernels.cuh"
@@ -165,7 +166,7 @@ struct hprmat_b200_ctx {
   bool tc_trsm = true;       // U12 by the tensor cores from L11^-1 (else substitution)
   int panel_rpc_min = 32;    // fewest panel rows per CTA
   double growth_limit = 1e6;  // mixed path: pivot growth above which C(E) is factorised in FP64
-  bool panel_cluster = true;  // panels that fit in one 16-CTA cluster use panel_cluster_kernel
+  bool panel_cluster = true;  // panels that fit in one 16-CTA cluster use panel_reg_kernel
   signed char cluster_ok[2][17] = {};  // per element size (float2, double2) and cluster size:
                                        // 0 unknown, 1 schedulable, -1 not
   int gmres_m = 12;          // longest FGMRES cycle per outer step (<= kGmresMaxM)
@@ -579,7 +580,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   HPR_CUDA_TRY(cudaMemsetAsync(status, 0, SW_COUNT * sizeof(int), c->stream));
   const int G0 = std::min(c->nsm, std::max(1, (N + 31) / 32));
   TRY(c->stage.ensure((size_t)2 * G0 * NB * sizeof(T) + (size_t)NB * sizeof(unsigned long long) +
-                      (size_t)2 * NB * sizeof(T) + 256));
+                      (size_t)2 * NB * sizeof(T) + (size_t)NB * NB * sizeof(T) + 256));
   TRY(c->swaps.ensure((size_t)nsteps * kSwapStride * sizeof(int)));
   TRY(c->ipiv.ensure((size_t)N * sizeof(int) + 64));
   unsigned char* sp = c->stage.as<unsigned char>();
@@ -588,6 +589,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(sp);
   sp += (size_t)NB * sizeof(unsigned long long);
   T* rowj = reinterpret_cast<T*>(sp);
+  T* urows = rowj + 2 * NB;  // the register panel's pivot-row exchange, NB x NB
   unsigned* growth = reinterpret_cast<unsigned*>(status + SW_COUNT - 1);
 
   float* bop = nullptr;
@@ -781,21 +783,23 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     return after_panel(s, k0, ncols, sw);
   };
   auto pk = panel_kernel<T, NB, NT>;
-  auto pkc = panel_cluster_kernel<T, NB, NT>;
+  auto pkc = panel_reg_kernel<T, NB>;
   // the largest rows per CTA of a cluster panel (shared memory of the opt-in limit, less the
   // static arrays)
   int rpc_max_c = 0;
-  while (panel_cluster_smem<T>(rpc_max_c + 1, NB) + 4096 <= (size_t)c->smem_optin) ++rpc_max_c;
+  const size_t static_c = (sizeof(T) == sizeof(double2) ? 20 : 12) * 1024;
+  while (rpc_max_c < kRegPanelRows && panel_reg_smem<T, NB>(rpc_max_c + 1) + static_c <= (size_t)c->smem_optin)
+    ++rpc_max_c;
   auto cluster_fits = [&](int g) -> bool {  // can the GPU hold a cluster of g such CTAs
     signed char& ok = c->cluster_ok[sizeof(T) == sizeof(double2)][g];
     if (ok == 0) {
-      const size_t sm = panel_cluster_smem<T>(rpc_max_c, NB);
+      const size_t sm = panel_reg_smem<T, NB>(rpc_max_c);
       ok = -1;
       if (cudaFuncSetAttribute((const void*)pkc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
           set_smem(pkc, sm) == HPRMAT_B200_OK) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(g);
-        cfg.blockDim = dim3(NT);
+        cfg.blockDim = dim3(kRegPanelThreads);
         cfg.dynamicSmemBytes = sm;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -817,10 +821,14 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     const int m = N - k0;
     if (c->panel_cluster && rpc_max_c > 0 && m <= 16 * rpc_max_c) {
       // the whole panel in one cluster: as many CTAs as panel_rpc_min rows allow, at most 16
-      const int Gc = std::min(16, std::max((m + rpc_max_c - 1) / rpc_max_c, (m + c->panel_rpc_min - 1) / c->panel_rpc_min));
+      // (one CTA up to 128 rows: without the cluster's exchange a column is shorter)
+      const int Gc = m <= 128 && m <= rpc_max_c
+                         ? 1
+                         : std::min(16, std::max((m + rpc_max_c - 1) / rpc_max_c,
+                                                 (m + c->panel_rpc_min - 1) / c->panel_rpc_min));
       if (cluster_fits(Gc)) {
         const int rpcc = (m + Gc - 1) / Gc;
-        const size_t smc = panel_cluster_smem<T>(rpcc, NB);
+        const size_t smc = panel_reg_smem<T, NB>(rpcc);
         TRY(set_smem(pkc, smc));
         PanelArgs<T> pa;
         pa.W = W;
@@ -831,7 +839,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
         pa.rpc = rpcc;
         pa.G = Gc;
         pa.ipiv = c->ipiv.as<int>();
-        pa.cand_rows = nullptr;
+        pa.cand_rows = urows;
         pa.keys = nullptr;
         pa.rowj = nullptr;
         pa.status = status;
@@ -846,7 +854,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
         pa.lup_plane = c->lup_plane;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(Gc);
-        cfg.blockDim = dim3(NT);
+        cfg.blockDim = dim3(kRegPanelThreads);
         cfg.dynamicSmemBytes = smc;
         cfg.stream = c->stream;
         cudaLaunchAttribute at[1];

@@ -1,0 +1,43 @@
+"""The cluster panel of the LU (panel.cuh): dense solves at the edges of its row split, sub-panels
+and cluster sizes, against numpy's solution."""
+import numpy as np
+import pytest
+
+from hprmat_b200 import api
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(n, ties):
+    rng = np.random.default_rng(n)
+    if ties:  # many equal moduli: the pivot is the lowest such row
+        a = rng.integers(-1, 2, (n, n)) + 1j * rng.integers(-1, 2, (n, n)) + 0.01 * rng.uniform(-1, 1, (n, n))
+        a[:, : n // 2] = np.round(a[:, : n // 2])
+        a += 3.0 * np.sqrt(n) * np.roll(np.eye(n), n // 3, axis=0)
+        return a
+    return rng.uniform(-1, 1, (n, n)) + 1j * rng.uniform(-1, 1, (n, n))
+
+
+@pytest.mark.parametrize("ties", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 17, 31, 33, 63, 65, 127, 128, 129, 145, 161, 257, 511, 513, 1025, 2995])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_panel_row_and_column_edges(precision, n, ties):
+    """|A X - B| <= 8 n u |A| |X| elementwise maxima (u = 2^-53): the backward error of an LU with
+    partial pivoting on these matrices (growth of a few), and of the refined mixed solve."""
+    a = _matrix(n, ties)
+    b = np.random.default_rng(7 * n).uniform(-1, 1, (n, 3)) + 0j
+    with api.Context(precision=precision, max_refine=8, tol=1e-15) as ctx:
+        x = ctx.solve_linear(a, b, allow_unconverged=True)
+    r = np.abs(a @ x - b).max()
+    assert r <= 8 * n * 2.0 ** -53 * np.abs(a).sum(1).max() * np.abs(x).max()
+
+
+@pytest.mark.parametrize("n,col", [(5, 0), (40, 16), (130, 7), (130, 128), (300, 45), (600, 333)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_zero_column_is_reported(precision, n, col):
+    a = _matrix(n, False)
+    a[:, col] = 0.0
+    with api.Context(precision=precision) as ctx:
+        with pytest.raises(api.HprmatError):
+            ctx.solve_linear(a, np.ones((n, 1), complex))
+        assert ctx.last_stats["info"] == col + 1
