@@ -613,67 +613,121 @@ __global__ void __launch_bounds__(256) cgemv_update_kernel(int M, int N, int K, 
 }
 
 // -------------------------------------------------------------------------------------
-// Explicit inverses of the diagonal blocks, used by the triangular solves with many
-// right-hand sides (each block solve becomes a small dense product instead of a chain of
-// nb dependent steps).  blockIdx.x = step, blockIdx.y = 0: unit lower L11, 1: upper U11.
-// Output per step: inv[(2*s + y) * NB * NB], column-major NB x NB, zero outside the
-// triangle, explicit unit diagonal for L11^-1.  In-place column sweeps as LAPACK's
-// xTRTI2: lower from the last column backwards, upper from the first column onwards.
-template <typename T, int NB, int NT>
-__global__ void __launch_bounds__(NT) tri_inverse_kernel(const T* __restrict__ W, long ld, int N, int nb,
-                                                         T* inv) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S = reinterpret_cast<T*>(smem_raw);  // [NB][NB] column-major
-  T* tmp = S + NB * NB;                   // [NB]
-  const int s = blockIdx.x;
-  const bool upper = blockIdx.y == 1;
-  const int k0 = s * nb;
-  const int nc = min(nb, N - k0);
+// Inverse of one NB x NB triangle, 16 columns of it per CTA, by blocks of 16: X = T^-1 E_jb from
+//   X_ib = D_ib^-1 (E_ib - sum_k T_{ib,k} X_k),  ib = jb, jb + 1, .. (lower) or jb, jb - 1, .. (upper),
+// D_ib the diagonal blocks, whose inverses every CTA forms for itself, one column per thread.  The
+// CTAs of a triangle are independent, so a chain of 7 block steps of one SM each replaces the
+// column sweep over the whole triangle on one SM (128 columns with two block barriers each).
+// Tm: the triangle (column-major, ld; order nc, identity beyond it), of which the strict lower part
+// with a unit diagonal or the upper part is read.  The result (rows of all blocks, 16 columns) is left in X [NB][kTiLd], row-major, zero outside the
+// triangle.  256 threads.
+constexpr int kTiB = 16;
+constexpr int kTiLd = kTiB + 2;  // even: 16-byte pieces stay aligned
+template <typename T, int NB>
+__host__ __device__ constexpr size_t tri_block_smem() {  // T blocks, diagonal inverses, X, one block of sums
+  return ((size_t)(NB / kTiB) * (NB / kTiB + 1) / 2 * kTiB * kTiB + (size_t)NB * kTiB + (size_t)NB * kTiLd +
+          (size_t)kTiB * kTiLd) * sizeof(T);
+}
+template <typename T, int NB>
+__device__ T* tri_block_inverse(unsigned char* smem, bool upper, int jb, const T* __restrict__ Tm, long ld, int nc) {
+  constexpr int B = kTiB, nb = NB / B;
+  T* blk = reinterpret_cast<T*>(smem);              // blocks (ib, kb) of T, column-major B x B
+  T* dinv = blk + (size_t)nb * (nb + 1) / 2 * B * B;  // [nb][B][B] column-major
+  T* X = dinv + (size_t)NB * B;                     // [NB][kTiLd]
+  T* rhs = X + (size_t)NB * kTiLd;                  // [B][kTiLd]: (k, c)
   const int tid = threadIdx.x;
-  for (int idx = tid; idx < NB * NB; idx += NT) {
-    int i = idx % NB, j = idx / NB;
-    T v = czero<T>();
-    if (i < nc && j < nc) {
-      if ((!upper && i > j) || (upper && i <= j)) v = W[(size_t)(k0 + i) + (size_t)(k0 + j) * ld];
-      if (!upper && i == j) v.x = 1;
+  // the blocks of this chain: ib from jb to the triangle's end, kb between jb and ib
+  const int nchain = upper ? jb + 1 : nb - jb;
+  auto row_block = [&](int s) { return upper ? jb - s : jb + s; };
+  auto slot = [&](int si, int sk) { return blk + (size_t)(si * (si + 1) / 2 + sk) * B * B; };
+  // all copies in flight at once; thread (i, j) of every block
+  {
+    const int bi = tid % B, bj = tid / B;
+    for (int si = 0; si < nchain; ++si)
+      for (int sk = 0; sk <= si; ++sk) {
+        const int i = row_block(si) * B + bi, j = row_block(sk) * B + bj;
+        T* dst = slot(si, sk) + tid;
+        if (i < nc && j < nc) {
+          cp_async_elem(dst, Tm + (size_t)i + (size_t)j * ld);
+        } else {
+          T v = czero<T>();
+          if (i == j) v.x = 1;
+          *dst = v;
+        }
+      }
+  }
+  for (int t = tid; t < NB * kTiLd; t += 256) X[t] = czero<T>();
+  cp_async_wait_all();
+  __syncthreads();
+  // inverses of the diagonal blocks: thread (s, c) solves D_s x = e_c in registers
+  if (tid < nchain * B) {
+    const int s = tid / B, c = tid % B;
+    const T* D = slot(s, s);
+    T x[B];
+#pragma unroll
+    for (int i = 0; i < B; ++i) {
+      x[i] = czero<T>();
+      if (i == c) x[i].x = 1;
     }
-    if (i >= nc && i == j) v.x = 1;  // identity padding keeps the padded block invertible
-    S[idx] = v;
+    if (!upper) {
+#pragma unroll
+      for (int k = 0; k < B; ++k)
+#pragma unroll
+        for (int i = k + 1; i < B; ++i) cfms(x[i], D[k * B + i], x[k]);
+    } else {
+#pragma unroll
+      for (int k = B - 1; k >= 0; --k) {
+        const T d = D[k * B + k];
+        x[k] = cmul(x[k], (d.x == 0 && d.y == 0) ? czero<T>() : crecip(d));
+#pragma unroll
+        for (int i = 0; i < k; ++i) cfms(x[i], D[k * B + i], x[k]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < B; ++i) dinv[(size_t)s * B * B + c * B + i] = x[i];
   }
   __syncthreads();
-  if (!upper) {
-    for (int j = nc - 2; j >= 0; --j) {
-      for (int i = j + 1 + tid; i < nc; i += NT) tmp[i] = S[i + j * NB];
-      __syncthreads();
-      for (int i = j + 1 + tid; i < nc; i += NT) {
-        T acc = czero<T>();
-        for (int k = j + 1; k <= i; ++k) cfma(acc, S[i + k * NB], tmp[k]);  // S[i][i] = 1
-        acc.x = -acc.x;
-        acc.y = -acc.y;
-        S[i + j * NB] = acc;
-      }
-      __syncthreads();
+  // thread (i, c) forms entry (i, c) of every block of the chain
+  const int i = tid % B, c = tid / B;
+  X[(size_t)(row_block(0) * B + i) * kTiLd + c] = dinv[c * B + i];
+  __syncthreads();
+  for (int s = 1; s < nchain; ++s) {
+    T acc[2] = {czero<T>(), czero<T>()};
+    for (int k = 0; k < s; ++k) {
+      const T* L = slot(s, k);
+      const T* xk = X + (size_t)row_block(k) * B * kTiLd + c;
+#pragma unroll
+      for (int e = 0; e < B; ++e) cfms(acc[e & 1], L[e * B + i], xk[e * kTiLd]);
     }
-  } else {
-    for (int j = 0; j < nc; ++j) {
-      for (int i = tid; i <= j; i += NT) tmp[i] = S[i + j * NB];
-      __syncthreads();
-      T d = tmp[j];
-      T dinv = (d.x == 0 && d.y == 0) ? czero<T>() : crecip(d);
-      for (int i = tid; i < j; i += NT) {
-        T acc = czero<T>();
-        for (int k = i; k < j; ++k) cfma(acc, S[i + k * NB], tmp[k]);
-        acc = cmul(acc, dinv);
-        acc.x = -acc.x;
-        acc.y = -acc.y;
-        S[i + j * NB] = acc;
-      }
-      if (tid == 0) S[j + j * NB] = dinv;
-      __syncthreads();
-    }
+    rhs[i * kTiLd + c] = cadd(acc[0], acc[1]);
+    __syncthreads();
+    const T* D = dinv + (size_t)s * B * B + i;
+    T o[2] = {czero<T>(), czero<T>()};
+#pragma unroll
+    for (int e = 0; e < B; ++e) cfma(o[e & 1], D[e * B], rhs[e * kTiLd + c]);
+    X[(size_t)(row_block(s) * B + i) * kTiLd + c] = cadd(o[0], o[1]);
+    __syncthreads();
   }
-  T* out = inv + ((size_t)2 * s + (upper ? 1 : 0)) * NB * NB;
-  for (int idx = tid; idx < NB * NB; idx += NT) out[idx] = S[idx];
+  return X;
+}
+
+// Explicit inverses of the diagonal blocks, used by the triangular solves with many
+// right-hand sides (each block solve becomes a small dense product instead of a chain of
+// nb dependent steps).  Grid (steps, 2, NB / 16): blockIdx.y = 0: unit lower L11, 1: upper U11;
+// blockIdx.z: 16 columns of the inverse.  Output per step: inv[(2*s + y) * NB * NB], column-major
+// NB x NB, zero outside the triangle, explicit unit diagonal for L11^-1, identity beyond the order
+// of the last block.  Measured (NB = 128): 4 steps 203 -> 19 us, 24 steps 218 -> 30 us; against a
+// column sweep over each triangle on one SM.
+template <typename T, int NB>
+__global__ void __launch_bounds__(256) tri_inverse_kernel(const T* __restrict__ W, long ld, int N, T* inv) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int s = blockIdx.x, jb = blockIdx.z;
+  const bool upper = blockIdx.y == 1;
+  const int k0 = s * NB;
+  const int nc = min(NB, N - k0);
+  const T* X = tri_block_inverse<T, NB>(smem_raw, upper, jb, W + (size_t)k0 + (size_t)k0 * ld, ld, nc);
+  T* out = inv + ((size_t)2 * s + (upper ? 1 : 0)) * NB * NB + (size_t)jb * kTiB * NB;
+  for (int idx = threadIdx.x; idx < NB * kTiB; idx += 256) out[idx] = X[(size_t)(idx % NB) * kTiLd + idx / NB];
 }
 
 // One diagonal block of a triangular solve with many right-hand sides:
@@ -739,125 +793,33 @@ __global__ void __launch_bounds__(NB * CW) diag_apply_kernel(const T* __restrict
 
 // -------------------------------------------------------------------------------------
 // Tensor-core TRSM of the mixed path (U12 = L11^-1 P A12), in three steps per block step:
-//   l11_inverse_planes_kernel: Linv = L11^-1 (unit lower, one CTA, column sweeps as xTRTI2)
-//       written as the A-operand planes of (I - Linv), K-major rows;
+//   l11_inverse_planes_kernel: Linv = L11^-1 (unit lower) written as the A-operand planes of (I - Linv), K-major rows;
 //   swap_gather_kernel: applies the step's row interchanges to the columns right of the
 //       panel, leaving P A12 in rows k0.. of W and as B-operand planes (per column K-major);
 //   tc_update: C -= (I - Linv) (P A12) with C = those rows of W, i.e. C = Linv P A12 = U12;
 //   u12_split_kernel: U12 -> B-operand planes of the trailing update and the LU planes.
-// Inverse of the unit lower triangle L11 in shared memory by recursive blocking: the
-// diagonal blocks of (up to) 16 x 16 are inverted by one warp each, all at once (column
-// sweeps, as xTRTI2), then pairs of blocks are joined with
-//   [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1  C^-1]
-// until the whole NB x NB block is done.  Dynamic shared memory: (NB*NB + (NB/2)^2) float2.
-template <int NB, int NT>
-__global__ void __launch_bounds__(NT) l11_inverse_planes_kernel(const float2* __restrict__ W, long ld, int k0,
+// One CTA per 16 columns of L11^-1 (tri_block_inverse); 38 us per step with the recursive joins of
+// the whole block on one SM before, 13 us now.
+template <int NB>
+__global__ void __launch_bounds__(256) l11_inverse_planes_kernel(const float2* __restrict__ W, long ld, int k0,
                                                                  int ncols, float* planes, long plane) {
-  constexpr int B0 = NB < 16 ? NB : 16;
-  static_assert(NT >= 32 * (NB / B0), "one warp per diagonal block");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* S = reinterpret_cast<float2*>(smem_raw);  // [NB][NB] column-major, L11 -> L11^-1 in place
-  float2* T = S + NB * NB;                          // [NB/2][NB/2] scratch
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  for (int idx = tid; idx < NB * NB; idx += NT) {
-    int i = idx % NB, j = idx / NB;
-    float2 v = make_float2(0.f, 0.f);
-    if (i < ncols && j < ncols && i > j) v = W[(size_t)(k0 + i) + (size_t)(k0 + j) * ld];
-    if (i == j) v.x = 1.f;
-    S[idx] = v;
-  }
-  __syncthreads();
-  // level 0: warp w inverts the diagonal block [B0 w, B0 w + B0)
-  if (warp < NB / B0) {
-    const int b = B0 * warp;
-    const bool in = lane < B0;
-    for (int j = B0 - 2; j >= 0; --j) {
-      const float2 l = in ? S[(b + lane) + (b + j) * NB] : make_float2(0.f, 0.f);  // lane k: L[k][j]
-      float2 acc = make_float2(0.f, 0.f);
-      for (int k = j + 1; k < B0; ++k) {
-        float2 lk;
-        lk.x = __shfl_sync(0xffffffffu, l.x, k);
-        lk.y = __shfl_sync(0xffffffffu, l.y, k);
-        if (in && k <= lane) cfma(acc, S[(b + lane) + (b + k) * NB], lk);  // Linv[i][k], Linv[i][i] = 1
-      }
-      __syncwarp();
-      if (in && lane > j) S[(b + lane) + (b + j) * NB] = make_float2(-acc.x, -acc.y);
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  // join blocks of size h into blocks of size 2h; every thread computes 2 x 4 tiles of the
-  // h x h products, so that six shared-memory loads feed eight complex FMAs.  The zeros above
-  // the diagonal of S make the triangular ranges rectangular within a tile.
-  for (int h = B0; h < NB; h *= 2) {
-    const int npair = NB / (2 * h);
-    const int th = h / 2, tw = h / 4;  // tiles per pair: th x tw
-    // T = B * Ainv for every pair (B: rows [a+h, a+2h), cols [a, a+h); Ainv(k, j) = 0, k < j)
-    for (int t = tid; t < npair * th * tw; t += NT) {
-      const int pr = t / (th * tw), r = t % (th * tw);
-      const int i0 = 2 * (r % th), j0 = 4 * (r / th);
-      const int a = pr * 2 * h;
-      float2 acc[2][4];
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[u][q] = make_float2(0.f, 0.f);
-      for (int k = j0; k < h; ++k) {
-        const float2 b0 = S[(a + h + i0) + (a + k) * NB], b1 = S[(a + h + i0 + 1) + (a + k) * NB];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float2 v = S[(a + k) + (a + j0 + q) * NB];
-          cfma(acc[0][q], b0, v);
-          cfma(acc[1][q], b1, v);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) T[pr * h * h + (i0 + u) + (j0 + q) * h] = acc[u][q];
-    }
-    __syncthreads();
-    // B := -Cinv * T  (Cinv: rows/cols [a+h, a+2h), lower: Cinv(i, k) = 0 for k > i)
-    for (int t = tid; t < npair * th * tw; t += NT) {
-      const int pr = t / (th * tw), r = t % (th * tw);
-      const int i0 = 2 * (r % th), j0 = 4 * (r / th);
-      const int a = pr * 2 * h;
-      float2 acc[2][4];
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[u][q] = make_float2(0.f, 0.f);
-      for (int k = 0; k <= i0 + 1; ++k) {
-        const float2 c0 = S[(a + h + i0) + (a + h + k) * NB], c1 = S[(a + h + i0 + 1) + (a + h + k) * NB];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float2 v = T[pr * h * h + k + (j0 + q) * h];
-          cfma(acc[0][q], c0, v);
-          cfma(acc[1][q], c1, v);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          S[(a + h + i0 + u) + (a + j0 + q) * NB] = make_float2(-acc[u][q].x, -acc[u][q].y);
-    }
-    __syncthreads();
-  }
+  const int jb = blockIdx.x;
+  const float2* X = tri_block_inverse<float2, NB>(smem_raw, false, jb, W + (size_t)k0 + (size_t)k0 * ld, ld, ncols);
   // (I - Linv) as A-operand planes: row i, K index j contiguous
-  for (int idx = tid; idx < NB * NB; idx += NT) {
-    int j = idx % NB, i = idx / NB;
-    float2 v = S[i + j * NB];
+  for (int idx = threadIdx.x; idx < NB * kTiB; idx += 256) {
+    const int i = idx / kTiB, c = idx % kTiB, j = jb * kTiB + c;
+    const float2 v = X[(size_t)i * kTiLd + c];
     float2 d = make_float2((i == j ? 1.f : 0.f) - v.x, -v.y);
     if (i >= ncols || j >= ncols) d = make_float2(0.f, 0.f);
     float hr, lr, hi_, li;
     tf32_split(d.x, hr, lr);
     tf32_split(d.y, hi_, li);
-    planes[idx] = hr;
-    planes[plane + idx] = lr;
-    planes[2 * plane + idx] = hi_;
-    planes[3 * plane + idx] = li;
+    const size_t off = (size_t)i * NB + j;
+    planes[off] = hr;
+    planes[plane + off] = lr;
+    planes[2 * plane + off] = hi_;
+    planes[3 * plane + off] = li;
   }
 }
 

@@ -166,10 +166,10 @@ extern "C" int hprmat_b200_solve_linear_noalloc(const void* d_A, void* d_B, int 
                                                  W + (k0 + ncols) + (size_t)(k0 + ncols) * ld, ld);
     HPR_CUDA_TRY(cudaGetLastError());
   }
-  auto ik = tri_inverse_kernel<T, NB, NT>;
-  const size_t ism = ((size_t)NB * NB + NB) * sizeof(T);
+  auto ik = tri_inverse_kernel<T, NB>;
+  const size_t ism = tri_block_smem<T, NB>();
   if (ism > 48 * 1024) HPR_CUDA_TRY(cudaFuncSetAttribute(ik, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ism));
-  ik<<<dim3(nsteps, 2), NT, ism, st>>>(W, ld, N, NB, inv);
+  ik<<<dim3(nsteps, 2, NB / kTiB), 256, ism, st>>>(W, ld, N, inv);
   HPR_CUDA_TRY(cudaGetLastError());
   // forward and backward substitution
   constexpr int DCW = 2;

@@ -49,15 +49,6 @@ __host__ __device__ constexpr size_t panel_reg_smem(int rpc) {
   return ((size_t)NB * (size_t)(rpc | 1) + (NB - W) * W + 2) * sizeof(T);
 }
 
-// Asynchronous copy of one element from global to shared memory.
-__device__ __forceinline__ void cp_async_elem(float2* dst, const float2* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(tc::smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_elem(double2* dst, const double2* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 __device__ __forceinline__ uint32_t mapa_u32(uint32_t saddr, uint32_t rank) {
   uint32_t r;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));

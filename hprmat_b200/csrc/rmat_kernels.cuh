@@ -472,6 +472,14 @@ __global__ void f2d_kernel(const float2* __restrict__ src, long lds, double2* ds
   float2 v = src[(size_t)r + (size_t)col * lds];
   dst[(size_t)r + (size_t)col * ldd] = make_double2((double)v.x * s, (double)v.y * s);
 }
+__global__ void add_f2d_kernel(const float2* __restrict__ src, long lds, double2* dst, long ldd, int N) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int col = blockIdx.y;
+  if (r >= N) return;
+  const float2 v = src[(size_t)r + (size_t)col * lds];
+  double2* d = dst + (size_t)r + (size_t)col * ldd;
+  *d = make_double2(d->x + (double)v.x, d->y + (double)v.y);
+}
 __global__ void copy_d_kernel(const double2* __restrict__ src, long lds, double2* dst, long ldd, int N) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   const int col = blockIdx.y;

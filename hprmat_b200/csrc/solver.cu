@@ -620,11 +620,10 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     if (mixed && c->tc_trsm) {
       // L11^-1 (as I - L11^-1 operand planes), P A12 gathered, U12 by one tensor-core GEMM
       constexpr int CW = 32;
-      const size_t ism = ((size_t)NB * NB + (size_t)(NB / 2) * (NB / 2)) * sizeof(float2);
-      constexpr int NTI = 512;
-      auto ik = l11_inverse_planes_kernel<NB, NTI>;
+      const size_t ism = tri_block_smem<float2, NB>();
+      auto ik = l11_inverse_planes_kernel<NB>;
       TRY(set_smem(ik, ism));
-      ik<<<1, NTI, ism, c->stream>>>(reinterpret_cast<const float2*>(W), ld, k0, ncols, c->linv.as<float>(),
+      ik<<<NB / kTiB, 256, ism, c->stream>>>(reinterpret_cast<const float2*>(W), ld, k0, ncols, c->linv.as<float>(),
                                      (long)NB * NB);
       LAUNCH_CHECK();
       auto gk = swap_gather_kernel<NB, CW, NT>;
@@ -930,10 +929,10 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   // explicit inverses of the diagonal blocks for the solves
   {
     TRY(c->inv.ensure((size_t)2 * nsteps * NB * NB * sizeof(T)));
-    auto ik = tri_inverse_kernel<T, NB, NT>;
-    size_t ism = ((size_t)NB * NB + NB) * sizeof(T);
+    auto ik = tri_inverse_kernel<T, NB>;
+    const size_t ism = tri_block_smem<T, NB>();
     TRY(set_smem(ik, ism));
-    ik<<<dim3(nsteps, 2), NT, ism, c->stream>>>(W, ld, N, NB, c->inv.as<T>());
+    ik<<<dim3(nsteps, 2, NB / kTiB), 256, ism, c->stream>>>(W, ld, N, c->inv.as<T>());
     LAUNCH_CHECK();
   }
   c->wave_ready = false;
@@ -1322,7 +1321,19 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
       stats->surface_change = change;
       stats->residual_floor = floor_rel;
     }
-    if (!(rel >= c->opts.tol) && !(error_based && surf && rel > 0.0)) break;  // converged (also on rel == 0)
+    if (!(rel >= c->opts.tol) && !(error_based && surf && rel > 0.0)) {  // converged (also on rel == 0)
+      // A residual below tol bounds the error only by the condition number times it.  The residual
+      // of the last iterate is at hand, so one more solve with the factors (no residual after
+      // it) takes the error in R down by the factors' contraction, 30 and more.
+      if (surf && outer > 0 && rel > 0.0) {
+        d2f_kernel<<<gconv, 256, 0, c->stream>>>(V, ldv, X32, ldv, N, nullptr);
+        LAUNCH_CHECK();
+        TRY(lu_solve_tc(c, st, X32, ldv, nrhs));
+        add_f2d_kernel<<<gconv, 256, 0, c->stream>>>(X32, ldv, X64, ldx, N);
+        LAUNCH_CHECK();
+      }
+      break;
+    }
     if (surf && outer > 0) {
       // change = size of the last correction in R, i.e. the error of the previous iterate;
       // the last cycle reduced that error by about last_est, which predicts the error left.
