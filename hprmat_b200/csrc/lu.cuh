@@ -446,6 +446,92 @@ __global__ void __launch_bounds__(NT) trsm_lower_kernel(TrsmArgs<T> a) {
   }
 }
 
+// trsm_lower_kernel of the FP64 LU's block steps (NB = 64) with the right-hand sides in registers:
+// 4 lanes share a column, lane g holding rows 4 a + g in x[a].  A step broadcasts x_k within the
+// 4 lanes and updates the rows below; L11 is staged in shared memory once, and no block barrier
+// separates the steps (trsm_lower_kernel: one barrier and one L2 read of L's column per step, 41 us
+// for up to 4000 columns; here 17 us).  x moves one register down every 4 steps, so that the code of
+// 4 steps serves all 64.  The same operations in the same order as trsm_lower_kernel.
+constexpr int kTrsmCols = 32;  // columns per CTA of 128 threads
+constexpr int kTrsmNB = 64;
+constexpr int kTrsmLdL = kTrsmNB + 1;  // L11 by rows: the 4 lanes of a column read 4 rows of a column
+constexpr size_t kTrsmSmem = ((size_t)kTrsmNB * kTrsmLdL + 2 * (size_t)kTrsmCols * (kTrsmNB + 1)) * sizeof(double2);
+template <int NB>
+__global__ void __launch_bounds__(128) trsm_lower_f64_kernel(TrsmArgs<double2> a) {
+  constexpr int R = NB / 4, LDA = NB + 1;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* L = reinterpret_cast<double2*>(smem_raw);   // [i][k]
+  double2* A = L + (size_t)NB * kTrsmLdL;              // [column][row]
+  double2* E = A + (size_t)kTrsmCols * LDA;            // displaced rows
+  const int tid = threadIdx.x;
+  const int cb = a.c_begin + blockIdx.x * kTrsmCols;
+  const int ncw = min(kTrsmCols, a.c_end - cb);
+  if (ncw <= 0) return;
+  const int ncols = a.ncols;
+  const bool swap = a.mode != 2, solve = a.mode != 1;
+  const int ne = swap ? *a.n_extra : 0;
+  if (solve)
+    for (int idx = tid; idx < NB * NB; idx += 128) {
+      const int i = idx % NB, k = idx / NB;
+      if (i < ncols && k < i) cp_async_elem(L + i * kTrsmLdL + k, a.W + (size_t)(a.k0 + i) + (size_t)(a.k0 + k) * a.ld);
+      else L[i * kTrsmLdL + k] = czero<double2>();
+    }
+  for (int idx = tid; idx < ncw * NB; idx += 128) {
+    const int j = idx % NB, cc = idx / NB;
+    if (j < ncols)
+      cp_async_elem(A + cc * LDA + j, a.X + (size_t)(swap ? a.top_src[j] : a.k0 + j) + (size_t)(cb + cc) * a.ldx);
+    else
+      A[cc * LDA + j] = czero<double2>();
+  }
+  for (int idx = tid; idx < ncw * ne; idx += 128) {
+    const int e = idx % ne, cc = idx / ne;
+    cp_async_elem(E + cc * LDA + e, a.X + (size_t)a.extra_src[e] + (size_t)(cb + cc) * a.ldx);
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  for (int idx = tid; idx < ncw * ne; idx += 128) {
+    const int e = idx % ne, cc = idx / ne;
+    a.X[(size_t)a.extra_dst[e] + (size_t)(cb + cc) * a.ldx] = E[cc * LDA + e];
+  }
+  const int g = tid & 3, cc = tid >> 2;  // this thread's row class and column
+  double gmax = 0.0;
+  if (solve) {
+    double2* col = A + (size_t)min(cc, ncw - 1) * LDA;
+    double2 x[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) x[q] = col[4 * q + g];
+    for (int kb = 0; kb < R; ++kb) {  // x[q] holds row 4 (kb + q) + g
+      const double2* Lr = L + (size_t)(4 * kb + g) * kTrsmLdL + 4 * kb;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        // x_k, k = 4 kb + e, from lane e of the column
+        double2 xk;
+        xk.x = __shfl_sync(0xffffffffu, x[0].x, e, 4);
+        xk.y = __shfl_sync(0xffffffffu, x[0].y, e, 4);
+        if (g > e) cfms(x[0], Lr[e], xk);
+#pragma unroll
+        for (int q = 1; q < R; ++q)
+          if (kb + q < R) cfms(x[q], Lr[(size_t)4 * q * kTrsmLdL + e], xk);
+      }
+      if (cc < ncw) col[4 * kb + g] = x[0];
+#pragma unroll
+      for (int q = 0; q + 1 < R; ++q) x[q] = x[q + 1];
+    }
+    __syncthreads();
+  }
+  for (int idx = tid; idx < ncw * NB; idx += 128) {
+    const int j = idx % NB, c = idx / NB;
+    if (j >= ncols) continue;
+    const double2 v = A[c * LDA + j];
+    a.X[(size_t)(a.k0 + j) + (size_t)(cb + c) * a.ldx] = v;
+    gmax = fmax(gmax, cabs1(v));
+  }
+  if (a.growth_bits && solve) {
+    for (int o = 16; o > 0; o >>= 1) gmax = fmax(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
+    if ((tid & 31) == 0) atomicMax(a.growth_bits, mag_hi(gmax));
+  }
+}
+
 // dst[i + j ldd] = W[src(i) + (col0 + j) ld], i < nr, j < ncol, src(i) = rows[i] (or row0 + i
 // without a row list): a block of W, optionally with its rows gathered.
 template <typename T>

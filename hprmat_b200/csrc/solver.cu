@@ -26,6 +26,7 @@
 #include "adjoint.cuh"
 #include "hessenberg.cuh"
 #include "rmat_kernels.cuh"
+#include "tri_solve.cuh"
 #include "tc_gemm.cuh"
 #include "tc_solve.cuh"
 #include "zgemm_f64.cuh"
@@ -163,6 +164,8 @@ struct hprmat_b200_ctx {
   int wave_sb = 0;        // blocks per diagonal super block of the scaled factors (1, 2, 4; 0: auto)
   int wave_sb_ready = 1;  // the value the current factors were prepared with
   bool wave_enabled = true;  // wavefront solves (else block-step solves)
+  bool inv_ready = false;    // explicit inverses of the current factors (tri_solve.cuh)
+  DevBuf invm, invy;         // L^-1 and U^-1; the product with L^-1
   bool tc_trsm = true;       // U12 by the tensor cores from L11^-1 (else substitution)
   int panel_rpc_min = 32;    // fewest panel rows per CTA
   double growth_limit = 1e6;  // mixed path: pivot growth above which C(E) is factorised in FP64
@@ -490,6 +493,50 @@ static int wave_prepare(hprmat_b200_ctx* c, const LUState& st) {
   return HPRMAT_B200_OK;
 }
 
+// Orders whose solves use explicit inverses of the whole factors (tri_solve.cuh): up to
+// kInvMaxSteps blocks of 128.  Whole rmatrix calls (seeded production potentials), wavefront
+// against inverses: N = 400 1.92 / 1.49 ms, 720 2.95 / 2.35, 992 3.71 / 3.16, 1240 4.65 / 4.04,
+// 1743 6.18 / 6.21, 1980 8.89 / 8.92: the inverses' N^3 passes what the sweeps cost near 14 blocks.
+// Refinement iterations are the same on both sides.
+constexpr int kInvMaxSteps = 10;
+
+static int inv_prepare(hprmat_b200_ctx* c, const LUState& st, const float2* W) {
+  const int N = st.N, ns = st.nsteps;
+  const long sig_ld = (N + 3) / 4 * 4;
+  TRY(c->wsig.ensure((size_t)ns * sig_ld * sizeof(int)));
+  TRY(c->wperm.ensure((size_t)3 * N * sizeof(int) + 64));
+  int* work = c->wperm.as<int>();
+  if (wave_perm_chain(c->swaps.as<int>(), kSwapStride, N, ns, work, c->wsig.as<int>(), sig_ld, work + 2 * (size_t)N,
+                      c->stream))
+    return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
+  ++c->launches;
+  TRY(c->invm.ensure((size_t)2 * st.ld * N * sizeof(float2)));
+  const InvArgs a{W, st.ld, c->inv.as<float2>(), c->wsig.as<int>(), sig_ld, N, c->invm.as<float2>(), st.ld};
+  const size_t sm = full_inverse_smem(N);
+  TRY(set_smem(full_inverse_kernel, sm));
+  full_inverse_kernel<<<dim3(cdiv_u(N, kInvCols), 2), 256, sm, c->stream>>>(a);
+  LAUNCH_CHECK();
+  c->inv_ready = true;
+  return HPRMAT_B200_OK;
+}
+
+// X <- U^-1 (L^-1 (P X)) with the explicit inverses.
+static int lu_solve_inv(hprmat_b200_ctx* c, const LUState& st, float2* X, long ldx, int nrhs) {
+  const int N = st.N;
+  TRY(c->invy.ensure((size_t)st.ld * nrhs * sizeof(float2)));
+  const float2* Li = c->invm.as<float2>();
+  const int* perm0 = c->wperm.as<int>() + 2 * (size_t)N;
+  const size_t sm = inv_apply_smem(N);
+  TRY(set_smem(inv_apply_kernel, sm));
+  const dim3 g(cdiv_u(N, 32), cdiv_u(nrhs, kInvCols));
+  inv_apply_kernel<<<g, 256, sm, c->stream>>>(Li, st.ld, N, false, perm0, X, ldx, nrhs, c->invy.as<float2>(), st.ld);
+  LAUNCH_CHECK();
+  inv_apply_kernel<<<g, 256, sm, c->stream>>>(Li + (size_t)st.ld * N, st.ld, N, true, nullptr, c->invy.as<float2>(),
+                                              st.ld, nrhs, X, ldx);
+  LAUNCH_CHECK();
+  return HPRMAT_B200_OK;
+}
+
 // X (N x nrhs, FP32 complex, ldx) <- (LU)^-1 P X with the prepared factors: right-hand side
 // planes of P X, forward sweep into the Y planes, backward sweep into X.
 static int lu_solve_wave(hprmat_b200_ctx* c, const LUState& st, float2* X, long ldx, int nrhs) {
@@ -613,6 +660,37 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     }
   }
 
+  // interchanges and / or forward substitution of a step (TrsmArgs::mode) on columns c_begin .. c_end
+  auto trsm = [&](int k0, int ncols, const StepSwaps& sw, int c_begin, int c_end, int mode) -> int {
+    if (c_end <= c_begin) return HPRMAT_B200_OK;
+    TrsmArgs<T> ta{};
+    ta.W = W;
+    ta.ld = ld;
+    ta.k0 = k0;
+    ta.ncols = ncols;
+    ta.top_src = sw.top_src;
+    ta.extra_dst = sw.extra_dst;
+    ta.extra_src = sw.extra_src;
+    ta.n_extra = sw.n_extra;
+    ta.X = W;
+    ta.ldx = ld;
+    ta.c_begin = c_begin;
+    ta.c_end = c_end;
+    ta.growth_bits = growth;
+    ta.mode = mode;
+    if constexpr (std::is_same<T, double2>::value && NB == kTrsmNB) {
+      TRY(set_smem(trsm_lower_f64_kernel<NB>, kTrsmSmem));
+      trsm_lower_f64_kernel<NB><<<cdiv_u(c_end - c_begin, kTrsmCols), 128, kTrsmSmem, c->stream>>>(ta);
+    } else {
+      constexpr int CW = 32;
+      auto tk = trsm_lower_kernel<T, NB, CW, NT>;
+      const size_t tsm = (size_t)CW * (NB + 1) * sizeof(T) + (size_t)CW * NB * sizeof(T);
+      TRY(set_smem(tk, tsm));
+      tk<<<cdiv_u(c_end - c_begin, CW), NT, tsm, c->stream>>>(ta);
+    }
+    LAUNCH_CHECK();
+    return HPRMAT_B200_OK;
+  };
   // after the panel of step s: row interchanges, U12 = L11^-1 P A12 and the trailing update
   auto after_panel = [&](int s, int k0, int ncols, const StepSwaps& sw) -> int {
     (void)s;
@@ -643,6 +721,8 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
                                                              k0 + ncols, N, bop, plane, c->lup.as<float>(),
                                                              c->lup_ld, c->lup_plane, growth);
       LAUNCH_CHECK();
+    } else if (!mixed) {
+      TRY(trsm(k0, ncols, sw, k0 + ncols, N, 0));
     } else {
       constexpr int CW = 32;
       auto tk = trsm_lower_kernel<T, NB, CW, NT>;
@@ -662,14 +742,13 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
       ta.c_begin = k0 + ncols;
       ta.c_end = N;
       ta.growth_bits = growth;
-      if (mixed) {  // U12 also as the B operand of the trailing update and into the LU planes
-        ta.bop = bop;
-        ta.bop_plane = plane;
-        ta.bop_col0 = k0 + ncols;
-        ta.lup = c->lup.as<float>();
-        ta.lup_ld = c->lup_ld;
-        ta.lup_plane = c->lup_plane;
-      }
+      // U12 also as the B operand of the trailing update and into the LU planes
+      ta.bop = bop;
+      ta.bop_plane = plane;
+      ta.bop_col0 = k0 + ncols;
+      ta.lup = c->lup.as<float>();
+      ta.lup_ld = c->lup_ld;
+      ta.lup_plane = c->lup_plane;
       tk<<<cdiv_u(N - k0 - ncols, CW), NT, tsm, c->stream>>>(ta);
       LAUNCH_CHECK();
     }
@@ -716,31 +795,6 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   auto step_swaps = [&](int s) {
     int* swb = c->swaps.as<int>() + (size_t)s * kSwapStride;
     return StepSwaps{swb, swb + kMaxNB, swb + 2 * kMaxNB, swb + 3 * kMaxNB};
-  };
-  auto trsm = [&](int k0, int ncols, const StepSwaps& sw, int c_begin, int c_end, int mode) -> int {
-    if (c_end <= c_begin) return HPRMAT_B200_OK;
-    constexpr int CW = 32;
-    auto tk = trsm_lower_kernel<T, NB, CW, NT>;
-    const size_t tsm = (size_t)CW * (NB + 1) * sizeof(T) + (size_t)CW * NB * sizeof(T);
-    TRY(set_smem(tk, tsm));
-    TrsmArgs<T> ta{};
-    ta.W = W;
-    ta.ld = ld;
-    ta.k0 = k0;
-    ta.ncols = ncols;
-    ta.top_src = sw.top_src;
-    ta.extra_dst = sw.extra_dst;
-    ta.extra_src = sw.extra_src;
-    ta.n_extra = sw.n_extra;
-    ta.X = W;
-    ta.ldx = ld;
-    ta.c_begin = c_begin;
-    ta.c_end = c_end;
-    ta.growth_bits = growth;
-    ta.mode = mode;
-    tk<<<cdiv_u(c_end - c_begin, CW), NT, tsm, c->stream>>>(ta);
-    LAUNCH_CHECK();
-    return HPRMAT_B200_OK;
   };
   auto pair_first = [&](int s, int k0) -> int {  // after panel s: the next panel's columns
     const int k1 = k0 + NB;
@@ -936,8 +990,13 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     LAUNCH_CHECK();
   }
   c->wave_ready = false;
+  c->inv_ready = false;
   if constexpr (NB == 128 && std::is_same<T, float2>::value) {
-    if (mixed && nsteps >= 2 && c->wave_enabled) TRY(wave_prepare(c, st));
+    // small orders: explicit inverses (unless the super block size was set by hand)
+    if (mixed && nsteps >= 2 && c->wave_enabled) {
+      if (nsteps <= kInvMaxSteps && c->wave_sb == 0) TRY(inv_prepare(c, st, W));
+      else TRY(wave_prepare(c, st));
+    }
   }
   HPR_CUDA_TRY(cudaMemcpyAsync(c->h_status, status, kStatusCopy * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -1040,6 +1099,7 @@ static int lu_solve_impl(hprmat_b200_ctx* c, const T* W, const LUState& st, T* X
 template <int NB>
 static int lu_solve_tc_impl(hprmat_b200_ctx* c, const LUState& st, float2* X, long ldx, int nrhs) {
   if (NB == 128 && c->wave_ready) return lu_solve_wave(c, st, X, ldx, nrhs);
+  if (NB == 128 && c->inv_ready) return lu_solve_inv(c, st, X, ldx, nrhs);
   const int N = st.N;
   const float2* inv = c->inv.as<float2>();
   constexpr int DCW = 2;
