@@ -2595,13 +2595,14 @@ static int scan_check_blocks(int nblocks, const hprmat_b200_scan_block* blocks, 
 // The blocks' potentials on the device (c->scan_cpot), once per block.
 static int scan_upload(hprmat_b200_ctx* c, int nblocks, const hprmat_b200_scan_block* blocks) {
   HPR_CUDA_TRY(cudaSetDevice(c->device));
-  c->scan_cpot.clear();
+  // the buffers stay with the context: freeing them made each scan wait for the device, and now and
+  // then for the driver (0.1 to 0.5 s next to the gigabytes of a shifted scan)
+  while ((int)c->scan_cpot.size() < nblocks) c->scan_cpot.emplace_back(new DevBuf());
   for (int b = 0; b < nblocks; ++b) {
     const hprmat_b200_scan_block& B = blocks[b];
     const size_t pbytes = (size_t)B.ncp1 * B.nch * B.nch * sizeof(double2);
-    c->scan_cpot.emplace_back(new DevBuf());
-    TRY(c->scan_cpot.back()->ensure(pbytes));
-    HPR_CUDA_TRY(cudaMemcpyAsync(c->scan_cpot.back()->p, B.cpot, pbytes, cudaMemcpyHostToDevice, c->stream));
+    TRY(c->scan_cpot[b]->ensure(pbytes));
+    HPR_CUDA_TRY(cudaMemcpyAsync(c->scan_cpot[b]->p, B.cpot, pbytes, cudaMemcpyHostToDevice, c->stream));
   }
   HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
   return HPRMAT_B200_OK;
