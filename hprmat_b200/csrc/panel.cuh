@@ -475,4 +475,423 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) panel_reg_kernel(PanelArg
   if (tid == 0 && a.growth_bits && s_growth > 0u) atomicMax(a.growth_bits, s_growth);
 }
 
+// ---------------------------------------------------------------- tall panels
+// A panel whose rows exceed one cluster's shared memory, in sub-panels of kSubW = 16 columns over
+// global memory (L2):
+//   panel_sub_kernel   one cluster of 16 CTAs factors 16 columns of all rows, as panel_reg_kernel does
+//                      (8 columns at a time in registers, RPT rows per thread); rows stay in place,
+//                      their positions in pos[] carry over from sub-panel to sub-panel;
+//   panel_rest_kernel  all SMs: U12 = L11^-1 A12 of the 16 pivot rows and the rank-16 update of the
+//                      panel's remaining columns; U12 goes to ubuf, the pivot rows stay as they were
+//                      (other CTAs read them);
+//   panel_planes_kernel, panel_place_kernel  after the last sub-panel: the L21 rows into the LU
+//                      planes, and the pivot and displaced rows to their final places.
+// Against panel_kernel (a grid barrier per column, 3.6-4.4 us): a column costs about 0.8 us, a
+// sub-panel's load, store and update 10-20 us more.  Measured, 128 columns FP32: 3100-6400 rows 500 ->
+// 320 us, 25600 rows 700 -> 570 us (a kernel per 1, 2, 3, 4 rows a thread: 30, 39, 47, 58 us a
+// sub-panel); the factorisation at N = 6400 28 -> 22.9 ms, 25600 357 -> 326 ms; FP64, N = 4000,
+// 20.0 -> 18.7 ms.  The same factors bit for bit.
+constexpr int kSubW = 16, kSubIW = 8;
+constexpr int kSubThreads = 512, kSubWarps = kSubThreads / 32;
+
+template <typename T>
+struct SubArgs {
+  T* W;
+  long ld;
+  int N, k0, ncols;      // the panel
+  int c0;                // first column of the sub-panel, panel-relative
+  int rpc, G;            // rows per CTA, CTAs (one cluster)
+  int* pos;              // [m] position of every row of the panel (written by c0 = 0)
+  int* prow;             // [NB] row that became pivot j
+  T* xrows;              // [kSubW][kSubW] exchange of the first half's pivot rows
+  T* ubuf;               // [NB][ldu] U rows right of their sub-panel
+  int ldu;
+  int* ipiv;
+  int* status;
+  StepSwaps sw;
+  unsigned* growth_bits;
+  float* lup;
+  long lup_ld, lup_plane;
+};
+
+template <typename T>
+__host__ __device__ constexpr size_t panel_sub_smem(int rpc) {
+  return (size_t)kSubW * (size_t)(rpc | 1) * sizeof(T) + 16;
+}
+
+template <typename T, int RPT>
+__global__ void __launch_bounds__(kSubThreads, 1) panel_sub_kernel(SubArgs<T> a) {
+  constexpr int NT = kSubThreads, W = kSubW, IW = kSubIW;
+  using PK = PivotKey<T>;
+  constexpr int kHead = sizeof(T) == sizeof(double2) ? 2 : 1;
+  constexpr int kMsg = kHead + IW * (int)sizeof(T) / 16;
+  constexpr int kPerSt = 32 / kMsg;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int m = a.N - a.k0;
+  const int G = a.G, b = (int)blockIdx.x;
+  const int r0 = b * a.rpc;
+  const int nloc = max(min(r0 + a.rpc, m) - r0, 0);
+  const int rpcp = a.rpc | 1;
+  T* P = reinterpret_cast<T*>(smem_raw);  // [W][rpcp]
+  __shared__ __align__(16) uint4 slot[2][kSubWarps][kMsg];
+  __shared__ __align__(16) uint4 rbuf[2][kMaxClusterCTAs][kMsg];
+  __shared__ __align__(16) T lu[W * W], u12[IW * IW];
+  __shared__ int s_prow[W], s_ipiv[W];
+  __shared__ uint64_t bar[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wc = min(W, a.ncols - a.c0);
+  const int FW = min(kSubWarps, (a.rpc + 31) / 32);
+  constexpr uint32_t kFull = 0xffffffffu;
+  constexpr uint32_t kMsgBytes = kMsg * 16;
+  if (tid == 0) {
+    tc::mbar_init(&bar[0], 1);
+    tc::mbar_init(&bar[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    tc::mbar_expect_tx(&bar[0], G * kMsgBytes);
+    if (wc > 1) tc::mbar_expect_tx(&bar[1], G * kMsgBytes);
+    if (b == 0 && a.c0 == 0) *a.sw.n_extra = 0;
+  }
+  if (tid < W) s_prow[tid] = -1;
+  for (int c = 0; c < wc; ++c) {
+    const T* src = a.W + (size_t)(a.k0 + r0) + (size_t)(a.k0 + a.c0 + c) * a.ld;
+    for (int lr = tid; lr < nloc; lr += NT) cp_async_elem(P + (size_t)c * rpcp + lr, src + lr);
+  }
+  int pos[RPT];
+  bool act[RPT], mine[RPT];
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int lr = tid + q * NT;
+    pos[q] = lr < nloc ? (a.c0 == 0 ? r0 + lr : a.pos[r0 + lr]) : 0;
+    mine[q] = act[q] = lr < nloc && pos[q] >= a.c0;
+  }
+  const int sd = lane / kMsg, sp = lane % kMsg;
+  constexpr int kSends = (kMaxClusterCTAs + kPerSt - 1) / kPerSt;
+  uint32_t rdst[kSends], rbar[kSends];
+#pragma unroll
+  for (int i = 0; i < kSends; ++i) {
+    const int d = sd + kPerSt * (warp + FW * i);
+    const bool to = sd < kPerSt && warp < FW && d < G;
+    rdst[i] = to ? mapa_u32(tc::smem_u32(&rbuf[0][b][sp]), (uint32_t)d) : 0u;
+    rbar[i] = to ? mapa_u32(tc::smem_u32(&bar[0]), (uint32_t)d) : 0u;
+  }
+  cp_async_wait_all();
+  cluster_arrive();
+  cluster_wait();
+  __syncthreads();
+  bool alive = true;
+  for (int pc = 0; pc < wc; pc += IW) {
+    const int wp = min(IW, wc - pc);
+    if (warp < FW) {
+      T v[RPT][IW], u[IW], l[RPT], v0[RPT];
+      bool upd[RPT];
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+#pragma unroll
+        for (int c = 0; c < IW; ++c)
+          v[q][c] = (act[q] && c < wp) ? P[(size_t)(pc + c) * rpcp + tid + q * NT] : czero<T>();
+        l[q] = czero<T>();
+        v0[q] = v[q][0];
+        upd[q] = false;
+      }
+      bool held[RPT];  // rows that take part in this half
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) held[q] = act[q];
+#pragma unroll
+      for (int c = 0; c < IW; ++c) u[c] = czero<T>();
+      T* pcol = P + (size_t)pc * rpcp + tid;
+      for (int j = 0; j < wp; ++j, pcol += rpcp) {
+        const int jl = pc + j, jj = a.c0 + jl, par = jl & 1;
+        uint2 key = make_uint2(0u, 0u);
+        int bq = 0;
+        T vb = v0[0];
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+          const uint2 kq = act[q] ? PK::key2(v0[q], pos[q]) : make_uint2(0u, 0u);
+          if (kq.y > key.y || (kq.y == key.y && kq.x > key.x)) {
+            key = kq;
+            bq = q;
+            vb = v0[q];
+          }
+        }
+        const unsigned mh = __reduce_max_sync(kFull, key.y);
+        const T inv = pivot_recip(vb);
+        if (j > 0) {
+#pragma unroll
+          for (int q = 0; q < RPT; ++q) {
+            if (upd[q]) {
+#pragma unroll
+              for (int c = 2; c < IW; ++c) {
+                T t = v[q][c];
+                cfms(t, l[q], u[c]);
+                v[q][c - 1] = t;
+              }
+            } else {
+#pragma unroll
+              for (int c = 2; c < IW; ++c) v[q][c - 1] = v[q][c];
+            }
+            v[q][0] = v0[q];
+          }
+        }
+        const int wl = winner_lane(key, mh);
+        uint4* sl = slot[par][warp];
+        if (lane == wl) {
+          store_head(sl, key, inv);
+#pragma unroll
+          for (int q = 0; q < RPT; ++q)
+            if (bq == q) store_row<IW>(sl + kHead, v[q]);
+        }
+        asm volatile("bar.sync 1, %0;" ::"r"(FW * 32) : "memory");
+        const uint4* won;
+        {
+          const uint2 k = lane < FW ? *reinterpret_cast<const uint2*>(&slot[par][lane][0]) : make_uint2(0u, 0u);
+          won = slot[par][winner_lane(k, __reduce_max_sync(kFull, k.y))];
+        }
+        {
+          const uint4 piece = won[sp];
+#pragma unroll
+          for (int i = 0; i < kSends; ++i) {
+            if (FW * i * kPerSt >= G) break;
+            if (rbar[i]) st_async16(rdst[i] + par * (uint32_t)sizeof(rbuf[0]), piece, rbar[i] + par * 8u);
+          }
+          if (alive) {
+            unsigned it = 0;
+            while (!tc::mbar_try_wait(&bar[par], (uint32_t)(jl >> 1) & 1u))
+              if (++it >= (1u << 22)) {
+                atomicExch(a.status + SW_TIMEOUT, 3);
+                alive = false;
+                break;
+              }
+          }
+          const uint2 k = lane < G ? *reinterpret_cast<const uint2*>(&rbuf[par][lane][0]) : make_uint2(0u, 0u);
+          won = rbuf[par][winner_lane(k, __reduce_max_sync(kFull, k.y))];
+        }
+        uint2 wk;
+        T winv;
+        load_head(won, wk, winv);
+        load_row<IW>(won + kHead, u);
+        const int p = PK::row2(wk);
+#pragma unroll
+        for (int q = 0; q < RPT; ++q) {
+          upd[q] = act[q] && pos[q] != p;
+          l[q] = v[q][0];
+          if (upd[q]) l[q] = cmul(l[q], winv);
+          v0[q] = v[q][1];
+          if (upd[q]) {
+            cfms(v0[q], l[q], u[1]);
+            if (pos[q] == jj) pos[q] = p;
+          } else if (act[q]) {  // this row is the pivot: final
+            act[q] = false;
+            pos[q] = jj;
+            s_prow[jl] = tid + q * NT;
+          }
+          if (held[q]) pcol[q * NT] = l[q];
+        }
+        s_ipiv[jl] = p;  // every thread the same value
+        if (tid == 0 && jl + 2 < wc) tc::mbar_expect_tx(&bar[par], G * kMsgBytes);
+      }
+    }
+    __syncthreads();
+    if (pc + IW >= wc) break;
+    // the first half's pivot rows (L11 and the raw second half) to every CTA
+    for (int idx = tid; idx < IW * W; idx += NT) {
+      const int j = idx / W, c = idx % W;
+      const int pr = s_prow[pc + j];
+      if (pr >= 0) __stcg(a.xrows + idx, P[(size_t)c * rpcp + pr]);
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (tid < IW * W) lu[tid] = __ldcg(a.xrows + tid);
+    __syncthreads();
+    if (tid < IW) {  // U12, one column per thread
+      T x[IW];
+#pragma unroll
+      for (int j = 0; j < IW; ++j) x[j] = lu[j * W + IW + tid];
+#pragma unroll
+      for (int k = 0; k < IW - 1; ++k)
+#pragma unroll
+        for (int j = k + 1; j < IW; ++j) cfms(x[j], lu[j * W + k], x[k]);
+#pragma unroll
+      for (int j = 0; j < IW; ++j) {
+        u12[j * IW + tid] = x[j];
+        const int pr = s_prow[pc + j];
+        if (pr >= 0) P[(size_t)(IW + tid) * rpcp + pr] = x[j];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      if (!act[q]) continue;
+      T* pr = P + tid + q * NT;
+      T lr[IW];
+#pragma unroll
+      for (int k = 0; k < IW; ++k) lr[k] = pr[(size_t)k * rpcp];
+#pragma unroll
+      for (int c = 0; c < IW; ++c) {
+        if (IW + c >= wc) break;
+        T t = pr[(size_t)(IW + c) * rpcp];
+#pragma unroll
+        for (int k = 0; k < IW; ++k) cfms(t, lr[k], u12[k * IW + c]);
+        pr[(size_t)(IW + c) * rpcp] = t;
+      }
+    }
+    // (a thread's own rows; the next half's loads are its own too)
+  }
+  cluster_arrive();
+  cluster_wait();
+  // the sub-panel back in place, positions, pivots
+#pragma unroll
+  for (int q = 0; q < RPT; ++q) {
+    const int lr = tid + q * NT;
+    if (lr >= nloc) continue;
+    if (mine[q]) {
+      T* dst = a.W + (size_t)(a.k0 + r0 + lr) + (size_t)(a.k0 + a.c0) * a.ld;
+#pragma unroll
+      for (int c = 0; c < W; ++c)
+        if (c < wc) dst[(size_t)c * a.ld] = P[(size_t)c * rpcp + lr];
+    }
+    a.pos[r0 + lr] = pos[q];
+    if (a.c0 + W >= a.ncols) {  // last sub-panel: the step's row interchanges
+      const int src = a.k0 + r0 + lr, dst = a.k0 + pos[q];
+      if (pos[q] < a.ncols) {
+        a.sw.top_src[pos[q]] = src;
+      } else if (dst != src) {
+        const int e = atomicAdd(a.sw.n_extra, 1);
+        a.sw.extra_dst[e] = dst;
+        a.sw.extra_src[e] = src;
+      }
+    }
+  }
+  if (tid < wc && s_prow[tid] >= 0) a.prow[a.c0 + tid] = r0 + s_prow[tid];
+  if (b == 0 && tid < wc) a.ipiv[a.k0 + a.c0 + tid] = a.k0 + s_ipiv[tid];
+}
+
+// 64 rows per CTA of 256 threads: 2 x 32 rows, four column groups.
+constexpr int kRestRows = 64;
+template <typename T, int NB>
+__global__ void __launch_bounds__(256) panel_rest_kernel(SubArgs<T> a) {
+  constexpr int W = kSubW;
+  __shared__ __align__(16) T lu[W * W];        // L11, column-major
+  __shared__ __align__(16) T Us[(NB > W ? NB - W : 1) * W];  // U12, W consecutive values per column
+  __shared__ int s_prow[W];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m = a.N - a.k0, c1 = a.c0 + W, rem = a.ncols - c1;
+  const int row = blockIdx.x * kRestRows + (warp & 1) * 32 + lane;
+  const bool on = row < m && a.pos[row] >= c1;
+  T l[W];
+  {  // this row's multipliers, in flight while U12 is formed
+    const T* src = a.W + (size_t)(a.k0 + min(row, m - 1)) + (size_t)(a.k0 + a.c0) * a.ld;
+#pragma unroll
+    for (int k = 0; k < W; ++k) l[k] = src[(size_t)k * a.ld];
+  }
+  if (tid < W) s_prow[tid] = a.prow[a.c0 + tid];
+  __syncthreads();
+  T x[W];
+  if (tid < rem) {
+    const T* src = a.W + (size_t)a.k0 + (size_t)(a.k0 + c1 + tid) * a.ld;
+#pragma unroll
+    for (int j = 0; j < W; ++j) x[j] = src[s_prow[j]];
+  }
+  {
+    const int j = tid % W, k = tid / W;
+    lu[k * W + j] = a.W[(size_t)(a.k0 + s_prow[j]) + (size_t)(a.k0 + a.c0 + k) * a.ld];
+  }
+  __syncthreads();
+  if (tid < rem) {
+#pragma unroll
+    for (int k = 0; k < W - 1; ++k) {
+      T lk[W];
+      load_row<W>(reinterpret_cast<const uint4*>(lu + k * W), lk);
+#pragma unroll
+      for (int j = k + 1; j < W; ++j) cfms(x[j], lk[j], x[k]);
+    }
+    store_row<W>(reinterpret_cast<uint4*>(Us + (size_t)tid * W), x);
+    if (blockIdx.x == 0)
+#pragma unroll
+      for (int j = 0; j < W; ++j) a.ubuf[(size_t)(a.c0 + j) * a.ldu + c1 + tid] = x[j];
+  }
+  __syncthreads();
+  if (!on) return;
+  T* dst = a.W + (size_t)(a.k0 + row) + (size_t)(a.k0 + c1) * a.ld;
+#pragma unroll 2
+  for (int c = warp >> 1; c < rem; c += 4) {
+    T v = dst[(size_t)c * a.ld];
+    T u[W];
+    load_row<W>(reinterpret_cast<const uint4*>(Us + (size_t)c * W), u);
+#pragma unroll
+    for (int k = 0; k < W; ++k) cfms(v, l[k], u[k]);
+    dst[(size_t)c * a.ld] = v;
+  }
+}
+
+// L21 rows (positions >= ncols) into the LU planes: 32 rows x 128 columns per CTA through shared
+// memory, so that both sides are coalesced.
+template <int NB>
+__global__ void __launch_bounds__(256) panel_planes_kernel(SubArgs<float2> a) {
+  __shared__ float2 tile[32][NB + 1];
+  __shared__ int s_pos[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m = a.N - a.k0, r0 = blockIdx.x * 32;
+  if (tid < 32) s_pos[tid] = r0 + tid < m ? a.pos[r0 + tid] : -1;
+  const float2* src = a.W + (size_t)(a.k0 + r0 + lane) + (size_t)a.k0 * a.ld;
+  if (r0 + lane < m)
+#pragma unroll 8
+    for (int c = warp; c < a.ncols; c += 8) tile[lane][c] = src[(size_t)c * a.ld];
+  __syncthreads();
+  for (int lr = warp; lr < 32; lr += 8) {
+    const int ps = s_pos[lr];
+    if (ps < a.ncols) continue;
+    float* dst = a.lup + (size_t)(a.k0 + ps) * a.lup_ld + a.k0;
+    for (int c = lane; c < a.ncols; c += 32) {
+      const float2 v = tile[lr][c];
+      float hr, lrr, hi_, li;
+      tf32_split(v.x, hr, lrr);
+      tf32_split(v.y, hi_, li);
+      dst[c] = hr;
+      dst[a.lup_plane + c] = lrr;
+      dst[2 * a.lup_plane + c] = hi_;
+      dst[3 * a.lup_plane + c] = li;
+    }
+  }
+}
+
+// Pivot rows (with their U columns from ubuf) and displaced rows to their final places, 8 columns
+// per CTA; max |u_ij| and zero pivots.  At most NB pivot rows and as many displaced ones.
+constexpr int kPlaceCols = 8;
+template <typename T, int NB>
+__global__ void __launch_bounds__(256) panel_place_kernel(SubArgs<T> a) {
+  using R = typename RealOf<T>::R;
+  __shared__ __align__(16) T tmp[kPlaceCols][2 * NB];
+  __shared__ int s_src[2 * NB], s_dst[2 * NB];
+  const int tid = threadIdx.x;
+  const int ne = *a.sw.n_extra, cnt = a.ncols + ne;
+  const int cb = blockIdx.x * kPlaceCols, nc = min(kPlaceCols, a.ncols - cb);
+  for (int i = tid; i < cnt; i += 256) {
+    s_src[i] = i < a.ncols ? a.sw.top_src[i] : a.sw.extra_src[i - a.ncols];
+    s_dst[i] = i < a.ncols ? a.k0 + i : a.sw.extra_dst[i - a.ncols];
+  }
+  __syncthreads();
+  unsigned g = 0u;
+  for (int idx = tid; idx < cnt * nc; idx += 256) {
+    const int i = idx % cnt, cc = idx / cnt, c = cb + cc;
+    T v;
+    if (i < a.ncols && c >= (i / kSubW + 1) * kSubW)
+      v = a.ubuf[(size_t)i * a.ldu + c];
+    else
+      v = a.W[(size_t)s_src[i] + (size_t)(a.k0 + c) * a.ld];
+    tmp[cc][i] = v;
+    if (c >= i) g = max(g, growth_key(v));
+    if (c == i && v.x == R(0) && v.y == R(0)) {  // zero pivot: the first one goes to info
+      const int col = a.k0 + c + 1;
+      if (atomicCAS(a.status + SW_INFO, 0, col) > col) atomicMin(a.status + SW_INFO, col);
+    }
+  }
+  __syncthreads();
+  for (int idx = tid; idx < cnt * nc; idx += 256) {
+    const int i = idx % cnt, cc = idx / cnt;
+    a.W[(size_t)s_dst[i] + (size_t)(a.k0 + cb + cc) * a.ld] = tmp[cc][i];
+  }
+  g = __reduce_max_sync(0xffffffffu, g);
+  if ((tid & 31) == 0 && g > 0u && a.growth_bits) atomicMax(a.growth_bits, growth_mag_hi<T>(g));
+}
+
 }  // namespace hprmat

@@ -179,6 +179,7 @@ struct hprmat_b200_ctx {
   long w_xld = 0, w_xplane = 0;
   bool wave_trace = false;
   DevBuf wtrace, ptrace;
+  DevBuf ppos;  // tall panels: row positions, pivot rows
   // the mixed factorisation held in W / lup / the wave buffers, for opts.reuse_factors: its
   // LUState (N, ld, nb, nsteps) and the channel block it belongs to
   bool lu_held = false;
@@ -924,6 +925,77 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
         ++c->launches;
         if (k0 + ncols >= N) break;
         TRY(after_step(s, k0, ncols, pa.sw));
+        continue;
+      }
+    }
+    if constexpr (NB >= 2 * kSubW) {
+      // a tall panel: sub-panels on one 16-CTA cluster, the rest of the panel on all SMs
+      const int rpt_max = sizeof(T) == sizeof(double2) ? 2 : 4;
+      const int rps = (m + 15) / 16;
+      const size_t ssm = panel_sub_smem<T>(rps);
+      const size_t sstatic = 16 * 1024;
+      if (c->panel_cluster && rps <= rpt_max * kSubThreads && ssm + sstatic <= (size_t)c->smem_optin &&
+          cluster_fits(16)) {
+        TRY(c->ppos.ensure((size_t)(N + NB) * sizeof(int)));
+        SubArgs<T> sa;
+        sa.W = W;
+        sa.ld = ld;
+        sa.N = N;
+        sa.k0 = k0;
+        sa.ncols = ncols;
+        sa.rpc = rps;
+        sa.G = 16;
+        sa.pos = c->ppos.as<int>();
+        sa.prow = sa.pos + N;
+        sa.xrows = cand_rows;  // the grid panel's exchange buffer: at least kSubW^2 elements
+        sa.ubuf = urows;
+        sa.ldu = NB;
+        sa.ipiv = c->ipiv.as<int>();
+        sa.status = status;
+        sa.sw = step_swaps(s);
+        sa.growth_bits = growth;
+        sa.lup = (mixed && k0 + ncols < N) ? c->lup.as<float>() : nullptr;
+        sa.lup_ld = c->lup_ld;
+        sa.lup_plane = c->lup_plane;
+        auto sub = [&](auto kern) -> int {
+          TRY(set_smem(kern, ssm));
+          HPR_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+          cudaLaunchConfig_t cfg = {};
+          cfg.gridDim = dim3(16);
+          cfg.blockDim = dim3(kSubThreads);
+          cfg.dynamicSmemBytes = ssm;
+          cfg.stream = c->stream;
+          cudaLaunchAttribute at[1];
+          at[0].id = cudaLaunchAttributeClusterDimension;
+          at[0].val.clusterDim.x = 16;
+          at[0].val.clusterDim.y = 1;
+          at[0].val.clusterDim.z = 1;
+          cfg.attrs = at;
+          cfg.numAttrs = 1;
+          HPR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, sa));
+          ++c->launches;
+          return HPRMAT_B200_OK;
+        };
+        const int rpt = (rps + kSubThreads - 1) / kSubThreads;
+        for (sa.c0 = 0; sa.c0 < ncols; sa.c0 += kSubW) {
+          if (rpt == 1) TRY(sub(panel_sub_kernel<T, 1>));
+          else if (rpt == 2) TRY(sub(panel_sub_kernel<T, 2>));
+          else if constexpr (sizeof(T) == sizeof(float2)) TRY(rpt == 3 ? sub(panel_sub_kernel<T, 3>) : sub(panel_sub_kernel<T, 4>));
+          if (sa.c0 + kSubW < ncols) {
+            panel_rest_kernel<T, NB><<<cdiv_u(m, kRestRows), 256, 0, c->stream>>>(sa);
+            LAUNCH_CHECK();
+          }
+        }
+        if constexpr (sizeof(T) == sizeof(float2)) {
+          if (sa.lup) {
+            panel_planes_kernel<NB><<<cdiv_u(m, 32), 256, 0, c->stream>>>(sa);
+            LAUNCH_CHECK();
+          }
+        }
+        panel_place_kernel<T, NB><<<cdiv_u(ncols, kPlaceCols), 256, 0, c->stream>>>(sa);
+        LAUNCH_CHECK();
+        if (k0 + ncols >= N) break;
+        TRY(after_step(s, k0, ncols, sa.sw));
         continue;
       }
     }

@@ -2,6 +2,7 @@
 and cluster sizes, against numpy's solution."""
 import numpy as np
 import pytest
+import torch
 
 from hprmat_b200 import api
 
@@ -41,3 +42,19 @@ def test_zero_column_is_reported(precision, n, col):
         with pytest.raises(api.HprmatError):
             ctx.solve_linear(a, np.ones((n, 1), complex))
         assert ctx.last_stats["info"] == col + 1
+
+
+@pytest.mark.parametrize("precision,n", [("mixed", 3010), ("mixed", 8192), ("mixed", 8209), ("mixed", 16400),
+                                         ("mixed", 24600), ("fp64", 3150), ("fp64", 8209)])
+def test_tall_panels(precision, n):
+    """Panels of more rows than a cluster's shared memory, at 1 to 4 rows per thread: random
+    matrices (pivots all over the rows), the bound of the test above on the GPU."""
+    gen = torch.Generator("cuda").manual_seed(n)
+    a = torch.complex(*(torch.rand((n, n), dtype=torch.float64, device="cuda", generator=gen) - 0.5 for _ in range(2)))
+    b = torch.rand((2, n), dtype=torch.float64, device="cuda", generator=gen).to(torch.complex128)
+    x, at = b.clone(), a.T.contiguous()
+    torch.cuda.synchronize()
+    with api.Context(precision=precision, max_refine=8, tol=1e-15) as ctx:
+        ctx.solve_linear_device(at.data_ptr(), x.data_ptr(), n, 2, allow_unconverged=True)
+    r = (a @ x.T - b.T).abs().max().item()
+    assert r <= 8 * n * 2.0 ** -53 * a.abs().sum(1).max().item() * x.abs().max().item()
