@@ -160,7 +160,7 @@ struct hprmat_b200_ctx {
   DevBuf wsig, wperm, wT, wdi, wbp, wyp, wxp, wflags, wdf1, wdf2, wptmp, wotmp;
   TcOperand op_wT, op_wdi, op_wbp, op_wyp, op_wxp;
   bool wave_ready = false;
-  int wave_un = 0;        // right-hand sides per unit (64, 128; 0: 128 when nrhs > 64)
+  int wave_un = 0;        // right-hand sides per unit (64, 128; 0: 64)
   int wave_sb = 0;        // blocks per diagonal super block of the scaled factors (1, 2, 4; 0: auto)
   int wave_sb_ready = 1;  // the value the current factors were prepared with
   bool wave_enabled = true;  // wavefront solves (else block-step solves)
@@ -542,7 +542,10 @@ static int lu_solve_inv(hprmat_b200_ctx* c, const LUState& st, float2* X, long l
 // planes of P X, forward sweep into the Y planes, backward sweep into X.
 static int lu_solve_wave(hprmat_b200_ctx* c, const LUState& st, float2* X, long ldx, int nrhs) {
   const int N = st.N, ns = st.nsteps;
-  const int un = c->wave_un > 0 ? c->wave_un : (nrhs > 64 ? 128 : 64);
+  // Units of 64 right-hand sides (one N = 128 operand of Re and Im) beat units of 128 at every order:
+  // refinement per iteration 0.53 / 0.60 ms at N = 1380, 0.65 / 0.88 at 3200, 1.04 / 1.37 at 6400,
+  // 1.78 / 2.48 at 12800 and 6.1 / 6.5 at 25600 (64 and 128 right-hand sides there).
+  const int un = c->wave_un > 0 ? c->wave_un : 64;
   const int G = (nrhs + un - 1) / un;
   const int npad = G * un;
   const long xld = (N + 3) / 4 * 4;
@@ -550,16 +553,17 @@ static int lu_solve_wave(hprmat_b200_ctx* c, const LUState& st, float2* X, long 
   // the TMA maps' box is un rows: a new unit width needs new maps even when npad is unchanged
   if (c->w_N != N || c->w_npad != npad || c->w_xld != xld || c->w_un != un || !c->wbp.p) {
     c->w_N = 0;
-    const size_t bytes = (size_t)4 * xplane * sizeof(float);
+    const int planes = wave_rhs_plane_count(un);
+    const size_t bytes = (size_t)planes * xplane * sizeof(float);
     TRY(c->wbp.ensure(bytes));
     TRY(c->wyp.ensure(bytes));
     TRY(c->wxp.ensure(bytes));
     HPR_CUDA_TRY(cudaMemsetAsync(c->wbp.p, 0, bytes, c->stream));
     HPR_CUDA_TRY(cudaMemsetAsync(c->wyp.p, 0, bytes, c->stream));
     HPR_CUDA_TRY(cudaMemsetAsync(c->wxp.p, 0, bytes, c->stream));
-    if (tc_make_operand(c->tcplan, c->op_wbp, c->wbp.as<float>(), N, npad, xld, xplane, un) ||
-        tc_make_operand(c->tcplan, c->op_wyp, c->wyp.as<float>(), N, npad, xld, xplane, un) ||
-        tc_make_operand(c->tcplan, c->op_wxp, c->wxp.as<float>(), N, npad, xld, xplane, un))
+    if (tc_make_operand(c->tcplan, c->op_wbp, c->wbp.as<float>(), N, npad, xld, xplane, un, planes) ||
+        tc_make_operand(c->tcplan, c->op_wyp, c->wyp.as<float>(), N, npad, xld, xplane, un, planes) ||
+        tc_make_operand(c->tcplan, c->op_wxp, c->wxp.as<float>(), N, npad, xld, xplane, un, planes))
       return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
     c->w_N = N;
     c->w_npad = npad;
@@ -584,7 +588,7 @@ static int lu_solve_wave(hprmat_b200_ctx* c, const LUState& st, float2* X, long 
     c->wtrace_units = ns * G;
     ws.trace = c->wtrace.as<long long>();
   }
-  if (wave_rhs_planes(X, ldx, perm0, N, nrhs, c->wbp.as<float>(), xld, xplane, c->stream) ||
+  if (wave_rhs_planes(X, ldx, perm0, N, nrhs, un, c->wbp.as<float>(), xld, xplane, c->stream) ||
       wave_sweep(c->tcplan, true, c->op_lu, c->op_wdi, c->op_wbp, c->op_wyp, ws, c->stream))
     return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
   ws.xp = c->wxp.as<float>();

@@ -286,16 +286,16 @@ int tc_gemm_init(TcGemmPlan& p, int device) {
 }
 
 int tc_make_operand(TcGemmPlan& p, TcOperand& op, const float* base, long kext, long rows, long ld, long plane,
-                    int box_rows) {
+                    int box_rows, int planes) {
   if (((uintptr_t)base & 15) || (ld % 4) || (plane % 4) || kext < 16 || rows < 1 || ld < kext ||
-      (box_rows != 64 && box_rows != 128 && box_rows != 256)) {
+      (box_rows != 64 && box_rows != 128 && box_rows != 256) || (planes != 4 && planes != 6)) {
     set_last_error_msg("tensor-core operand: misaligned or invalid view");
     return -1;
   }
   EncodeTiledFn enc = reinterpret_cast<EncodeTiledFn>(p.encode);
-  cuuint64_t dims[3] = {(cuuint64_t)kext, (cuuint64_t)rows, 4};
+  cuuint64_t dims[3] = {(cuuint64_t)kext, (cuuint64_t)rows, (cuuint64_t)planes};
   cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)plane * 4};
-  cuuint32_t box[3] = {(cuuint32_t)kKC, (cuuint32_t)box_rows, 4};
+  cuuint32_t box[3] = {(cuuint32_t)kKC, (cuuint32_t)box_rows, (cuuint32_t)planes};
   cuuint32_t es[3] = {1, 1, 1};
   CUresult r = enc(&op.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, es,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

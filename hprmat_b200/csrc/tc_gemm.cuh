@@ -26,7 +26,7 @@ struct TcOperand {
 
 int tc_gemm_init(TcGemmPlan& p, int device);
 int tc_make_operand(TcGemmPlan& p, TcOperand& op, const float* base, long kext, long rows, long ld, long plane,
-                    int box_rows);
+                    int box_rows, int planes = 4);  // planes: 4 or 6
 
 // C[M x Nc] -= A * B for complex C (float2, column-major, ldc).  Row m of A is operand row
 // a_row0 + m, K values a_k0 .. a_k0 + K - 1; column n of B is operand row b_row0 + n, K values

@@ -236,32 +236,14 @@ __global__ void __launch_bounds__(256) dinv_assemble_kernel(const float2* __rest
   }
 }
 
-// ------------------------------------------------------------------ right-hand side planes
-__global__ void __launch_bounds__(256) rhs_planes_kernel(const float2* __restrict__ X, long ldx,
-                                                          const int* __restrict__ perm0, int N, float* bp, long bld,
-                                                          long bplane) {
-  const int i = blockIdx.x * 256 + threadIdx.x;
-  const int c = blockIdx.y;
-  if (i >= N) return;
-  const float2 v = X[(size_t)perm0[i] + (size_t)c * ldx];
-  float hr, lr, hi, li;
-  tf32_split(v.x, hr, lr);
-  tf32_split(v.y, hi, li);
-  const size_t off = (size_t)c * bld + i;
-  bp[off] = hr;
-  bp[bplane + off] = lr;
-  bp[2 * bplane + off] = hi;
-  bp[3 * bplane + off] = li;
-}
-
 // ------------------------------------------------------------------ shared pieces of the
 // two tensor-core kernels below: a 3xTF32 complex MMA chain over K = 128 from a ring of
 // shared-memory stages, each stage one 16-deep K chunk of the A tile (4 planes x 128 rows)
 // and of the B tile (4 planes x BN rows).
-template <int BN>
+template <int BN, int BP = 4>  // BP: planes of the B tile
 struct Ring {
   static constexpr int kABytes = 4 * kNB * kKC * 4;
-  static constexpr int kBBytes = 4 * BN * kKC * 4;
+  static constexpr int kBBytes = BP * BN * kKC * 4;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStages = (192 * 1024) / kStageBytes;
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 1024;
@@ -286,12 +268,74 @@ __device__ __forceinline__ void mma_chunk(unsigned char* smem, int stage, uint32
   }
 }
 
+// The same product for 64 right-hand sides with Re and Im side by side in one N = 128 operand: an
+// MMA of N = 64 takes as long as one of N = 128 (64 cycles: the A tile's shared-memory reads), so
+// 6 MMAs per K-step of 8, D = [Re | Im] += Ar [Br | Bi] + Ai [-Bi | Br], do the work of 12.  The B
+// tile has six planes -Bi, Br, Bi (heads, then tails), so that both operands are windows of it.
+__device__ __forceinline__ void mma_chunk_wide(unsigned char* smem, int stage, uint32_t t_acc, bool first_chunk,
+                                               bool negate) {
+  using R = Ring<64, 6>;
+  constexpr uint32_t kPlane = 64 * 64;  // bytes of one B plane of a chunk
+  const uint32_t sa = smem_u32(smem + stage * R::kStageBytes);
+  const uint32_t sb = sa + R::kABytes;
+  const uint32_t id = idesc_tf32<128>(negate);
+#pragma unroll
+  for (int kk = 0; kk < kKC / 8; ++kk) {
+    const uint32_t off = kk * 32;
+    uint64_t a[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a[q] = sdesc_k_sw64(sa + q * (kNB * 64) + off);
+    const uint64_t ih = sdesc_k_sw64(sb + off), rh = sdesc_k_sw64(sb + kPlane + off);            // [-Bi|Br], [Br|Bi]
+    const uint64_t il = sdesc_k_sw64(sb + 3 * kPlane + off), rl = sdesc_k_sw64(sb + 4 * kPlane + off);
+    mma_tf32(t_acc, a[0], rl, id, (first_chunk && kk == 0) ? 0u : 1u);
+    mma_tf32(t_acc, a[1], rh, id, 1u);
+    mma_tf32(t_acc, a[2], il, id, 1u);
+    mma_tf32(t_acc, a[3], ih, id, 1u);
+    mma_tf32(t_acc, a[0], rh, id, 1u);
+    mma_tf32(t_acc, a[2], ih, id, 1u);
+  }
+}
+
+// Value v of right-hand side planes at d (planes `plane` floats apart): UN = 64 writes the six planes
+// of mma_chunk_wide, UN = 128 Re and Im as heads and tails.
+template <int UN>
+__device__ __forceinline__ void put_rhs_planes(float* d, size_t plane, float2 v) {
+  float hr, lr, hi, li;
+  tf32_split(v.x, hr, lr);
+  tf32_split(v.y, hi, li);
+  if (UN == 64) {
+    d[0] = -hi;
+    d[plane] = hr;
+    d[2 * plane] = hi;
+    d[3 * plane] = -li;
+    d[4 * plane] = lr;
+    d[5 * plane] = li;
+  } else {
+    d[0] = hr;
+    d[plane] = lr;
+    d[2 * plane] = hi;
+    d[3 * plane] = li;
+  }
+}
+
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 __device__ __forceinline__ long long globaltimer_ns() {
   long long t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
+}
+
+// ------------------------------------------------------------------ right-hand side planes
+template <int UN>
+__global__ void __launch_bounds__(256) rhs_planes_kernel(const float2* __restrict__ X, long ldx,
+                                                          const int* __restrict__ perm0, int N, float* bp, long bld,
+                                                          long bplane) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  const int c = blockIdx.y;
+  if (i >= N) return;
+  const float2 v = X[(size_t)perm0[i] + (size_t)c * ldx];
+  put_rhs_planes<UN>(bp + (size_t)c * bld + i, bplane, v);
 }
 
 // ------------------------------------------------------------------ off-diagonal scaling
@@ -529,7 +573,8 @@ template <int UN, bool FWD>
 __global__ void __launch_bounds__(kThreads, 1)
     wavefront_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmD,
                      const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmX, WaveArgs p) {
-  using R = Ring<UN>;
+  constexpr bool kWide = UN == 64;
+  using R = Ring<UN, kWide ? 6 : 4>;
   constexpr int kStages = R::kStages;
   constexpr int kSlots = 512 / (2 * UN);  // accumulators (Re + Im, 2 UN columns each)
   constexpr int kTmemCols = 512;
@@ -653,7 +698,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int kc = 0; kc < nch; ++kc) {
           if (!mbar_wait(&full[stage], phase, abort_flag, err, 64)) { ok = false; break; }
           tc_fence_after();
-          mma_chunk<UN>(smem, stage, t_re, t_im, first && kc == 0, negate);
+          if constexpr (kWide)
+            mma_chunk_wide(smem, stage, t_re, first && kc == 0, negate);
+          else
+            mma_chunk<UN>(smem, stage, t_re, t_im, first && kc == 0, negate);
           mma_commit(&empty[stage]);
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
@@ -727,14 +775,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int e = 0; e < 16; ++e) {
               const int col = h * UN + c_begin + 16 * (i0 + c) + e;
               if (rv && col < p.nrhs) {
-                float hr, lr, hi, li;
-                tf32_split(-re[c][e], hr, lr);
-                tf32_split(-im[c][e], hi, li);
-                float* d = p.xp + (size_t)col * p.xp_ld + row;
-                d[0] = hr;
-                d[p.xp_plane] = lr;
-                d[2 * p.xp_plane] = hi;
-                d[3 * p.xp_plane] = li;
+                put_rhs_planes<UN>(p.xp + (size_t)col * p.xp_ld + row, p.xp_plane, make_float2(-re[c][e], -im[c][e]));
               }
             }
           }
@@ -783,7 +824,7 @@ template <int UN, bool FWD>
 int launch_wave(TcGemmPlan& pl, const TcOperand& opM, const TcOperand& opD, const TcOperand& opB0,
                 const TcOperand& opX, const WaveArgs& args, int nunits, cudaStream_t s) {
   auto kern = wavefront_kernel<UN, FWD>;
-  const int smem = Ring<UN>::kSmemBytes;
+  const int smem = Ring<UN, UN == 64 ? 6 : 4>::kSmemBytes;
   HPR_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int grid = nunits < pl.nsm ? nunits : pl.nsm;
   CUtensorMap m = opM.map, d = opD.map, b0 = opB0.map, x = opX.map;
@@ -848,10 +889,13 @@ int wave_scale_offdiag(TcGemmPlan& pl, const TcOperand& opD, const TcOperand& op
   return 0;
 }
 
-int wave_rhs_planes(const float2* X, long ldx, const int* perm0, int N, int nrhs, float* bp, long bld, long bplane,
-                    cudaStream_t s) {
+int wave_rhs_planes(const float2* X, long ldx, const int* perm0, int N, int nrhs, int un, float* bp, long bld,
+                    long bplane, cudaStream_t s) {
   dim3 grid((N + 255) / 256, nrhs);
-  rhs_planes_kernel<<<grid, 256, 0, s>>>(X, ldx, perm0, N, bp, bld, bplane);
+  if (un == 64)
+    rhs_planes_kernel<64><<<grid, 256, 0, s>>>(X, ldx, perm0, N, bp, bld, bplane);
+  else
+    rhs_planes_kernel<128><<<grid, 256, 0, s>>>(X, ldx, perm0, N, bp, bld, bplane);
   HPR_CUDA_TRY(cudaGetLastError());
   return 0;
 }

@@ -58,9 +58,14 @@ int wave_dinv_double(const float2* dfh, int h, int nblk, const float* T, long ld
 int wave_scale_offdiag(TcGemmPlan& p, const TcOperand& opD, const TcOperand& opT, int N, int nsteps, int sb,
                        float* lup, long lup_ld, long lup_plane, cudaStream_t s);
 
-// B-operand planes of (P B): bp[p][c][i] = split(X[perm0[i] + c ldx]), i < N, c < nrhs.
-int wave_rhs_planes(const float2* X, long ldx, const int* perm0, int N, int nrhs, float* bp, long bld, long bplane,
-                    cudaStream_t s);
+// Planes of the right-hand sides and solutions by the unit width un: 64 takes six (-Im, Re, Im as
+// heads, then as tails; Re and Im are one N = 128 operand), 128 takes four (Re head and tail, Im
+// head and tail).
+inline int wave_rhs_plane_count(int un) { return un == 64 ? 6 : 4; }
+
+// B-operand planes of (P B): bp[p][c][i] from X[perm0[i] + c ldx], i < N, c < nrhs.
+int wave_rhs_planes(const float2* X, long ldx, const int* perm0, int N, int nrhs, int un, float* bp, long bld,
+                    long bplane, cudaStream_t s);
 
 struct WaveSolve {
   int N = 0, nsteps = 0, nrhs = 0;

@@ -51,10 +51,10 @@ int hprmat_b200_dev_counters(hprmat_b200_ctx* ctx, unsigned long long* launches,
                              int* tc_launches, int reset);
 
 /* Tuning knobs for benchmarks and experiments (defaults in parentheses):
-     "wave_un"        right-hand sides per unit of the wavefront solves: 64, 128 (0: 128 when
-                      nrhs > 64, else 64);
+     "wave_un"        right-hand sides per unit of the wavefront solves: 64, 128 (0: 64);
      "wave_sb"        blocks per diagonal super block of the solves' scaled factors: 1, 2, 4
-                      (0: 4, or 2 below 4 blocks); takes effect at the next factorisation;
+                      (0: 4, and explicit inverses of the whole factors up to 10 blocks); takes
+                      effect at the next factorisation;
      "wave"           wavefront solves on/off (1);
      "tc_trsm"        U12 by a tensor-core product with L11^-1 (1) or by substitution (0);
      "panel_rpc_min"  fewest panel rows per CTA (32);
