@@ -177,8 +177,11 @@ __global__ void surface_rhs_kernel(MeshDev mesh, T* X, long ldx, int N, double s
 //             K_c = tc - bloch_c blo0 + diag(fac_c / r_i^2 + kk_c)  (real, built per tile);
 //   coupling: batch i,  out[c*nr + i, col] -= sum_c' cpot(r_i, c, c') X[c'*nr + i, col]
 // (src/rmatrix_hp.F90:246-293 for the matrix they multiply by).  resid_tile_kernel: 256
-// threads compute a 64 x 64 tile (4 x 4 complex values each) from 16-deep K chunks staged in
+// threads compute a 64 x BN tile (4 x BN / 16 complex values each) from 16-deep K chunks staged in
 // shared memory; resid_tile2_kernel the compensated and modulus variants of the outer steps.
+// FP64-bound: BN = 16, 32 or 64 by the columns at hand (resid_bn), since 8 right-hand sides in a
+// 64-wide tile were 7/8 padding (N = 400: compensated kinetic 29 -> 13 us, plain 17 -> 14 us,
+// moduli, now formed once per element, 28 -> 8 us; N = 6400, 32 columns: 165 -> 94, 59 -> 46 us).
 struct KineticTile {
   MeshDev mesh;
   ChannelData ch;
@@ -227,9 +230,14 @@ struct CouplingTile {
   __device__ double2 init(int, int, int, const double2* out, size_t idx) const { return out[idx]; }
 };
 
-template <class Op, bool REAL_A>
+inline int resid_bn(int ncol) {
+  if (ncol <= 16) return 16;
+  return (ncol + 31) / 32 * 32 < (ncol + 63) / 64 * 64 ? 32 : 64;
+}
+
+template <class Op, bool REAL_A, int BN>
 __global__ void __launch_bounds__(256, 2) resid_tile_kernel(Op op, int M, int Ncol, int K, double2* out, long ldo) {
-  constexpr int BM = 64, BN = 64, BK = 16;
+  constexpr int BM = 64, BK = 16, QN = BN / 16;  // QN columns per thread
   using AT = typename std::conditional<REAL_A, double, double2>::type;
   __shared__ AT As[BK][BM];
   __shared__ double2 Bs[BK][BN + 1];
@@ -237,11 +245,11 @@ __global__ void __launch_bounds__(256, 2) resid_tile_kernel(Op op, int M, int Nc
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
-  double2 acc[4][4];
+  double2 acc[4][QN];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[r][q] = make_double2(0.0, 0.0);
+    for (int q = 0; q < QN; ++q) acc[r][q] = make_double2(0.0, 0.0);
   for (int k0 = 0; k0 < K; k0 += BK) {
     // A tile: consecutive threads along m
 #pragma unroll
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(256, 2) resid_tile_kernel(Op op, int M, int Nc
     }
     // B tile: consecutive threads along k
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
+    for (int e = 0; e < BN * BK / 256; ++e) {
       const int idx = tid + 256 * e;
       const int kk = idx % BK, nn = idx / BK;
       const int n = n0 + nn, k = k0 + kk;
@@ -267,15 +275,15 @@ __global__ void __launch_bounds__(256, 2) resid_tile_kernel(Op op, int M, int Nc
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       AT av[4];
-      double2 bv[4];
+      double2 bv[QN];
 #pragma unroll
       for (int r = 0; r < 4; ++r) av[r] = As[kk][tx + 16 * r];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) bv[q] = Bs[kk][ty + 16 * q];
+      for (int q = 0; q < QN; ++q) bv[q] = Bs[kk][ty + 16 * q];
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < QN; ++q) {
           if constexpr (REAL_A) {
             acc[r][q].x = fma(av[r], bv[q].x, acc[r][q].x);
             acc[r][q].y = fma(av[r], bv[q].y, acc[r][q].y);
@@ -292,7 +300,7 @@ __global__ void __launch_bounds__(256, 2) resid_tile_kernel(Op op, int M, int Nc
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < QN; ++q) {
       const int m = m0 + tx + 16 * r, n = n0 + ty + 16 * q;
       if (m < M && n < Ncol) {
         const size_t idx = op.o(z, m, n, ldo);
@@ -302,7 +310,7 @@ __global__ void __launch_bounds__(256, 2) resid_tile_kernel(Op op, int M, int Nc
     }
 }
 
-// The outer-step variants of the same products, 32 x 64 tiles (2 x 4 values per thread):
+// The outer-step variants of the same products, 32 x BN tiles (2 x BN / 16 values per thread):
 //   kComp1:  kinetic, out = B - K_c X with compensated (Dot2) sums; the low words go to lo;
 //   kComp2:  coupling, out = (out + lo) - V X with compensated sums, rounded once;
 //   kAbs1:   kinetic, out = |B| + |K_c| |X| (real part; the rounding scale of the residual);
@@ -311,10 +319,10 @@ enum ResidTileMode { kComp1 = 0, kComp2 = 1, kAbs1 = 2, kAbs2 = 3 };
 
 // Batched over units (energies): blockIdx.y = column tile + ytiles * unit; unit u works on
 // op.at(u) and on out, lo + u * so.
-template <class Op, bool REAL_A, int MODE>
+template <class Op, bool REAL_A, int MODE, int BN>
 __global__ void __launch_bounds__(256) resid_tile2_kernel(Op op_all, int M, int Ncol, int K, double2* out, long ldo,
                                                           double2* lo, int ytiles, long so) {
-  constexpr int BM = 32, BN = 64, BK = 16;
+  constexpr int BM = 32, BK = 16, QN = BN / 16;
   using AT = typename std::conditional<REAL_A, double, double2>::type;
   __shared__ AT As[BK][BM];
   __shared__ double2 Bs[BK][BN + 1];
@@ -326,12 +334,12 @@ __global__ void __launch_bounds__(256) resid_tile2_kernel(Op op_all, int M, int 
   const int m0 = blockIdx.x * BM, n0 = (blockIdx.y - unit * ytiles) * BN;
   const int tid = threadIdx.x;
   const int tx = tid & 15, ty = tid >> 4;
-  Acc2 sr[2][4], si[2][4];
-  double ar[2][4];
+  Acc2 sr[2][QN], si[2][QN];
+  double ar[2][QN];
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < QN; ++q) {
       ar[r][q] = 0.0;
       const int m = m0 + tx + 16 * r, n = n0 + ty + 16 * q;
       if (m < M && n < Ncol) {
@@ -360,29 +368,33 @@ __global__ void __launch_bounds__(256) resid_tile2_kernel(Op op_all, int M, int 
       if constexpr (REAL_A) {
         As[kk][mm] = (m < M && k < K) ? op.a(z, m, k) : 0.0;
       } else {
-        As[kk][mm] = (m < M && k < K) ? op.a(z, m, k) : make_double2(0.0, 0.0);
+        double2 v = (m < M && k < K) ? op.a(z, m, k) : make_double2(0.0, 0.0);
+        if (MODE == kAbs2) v = make_double2(hypot(v.x, v.y), 0.0);
+        As[kk][mm] = v;
       }
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
+    for (int e = 0; e < BN * BK / 256; ++e) {
       const int idx = tid + 256 * e;
       const int kk = idx % BK, nn = idx / BK;
       const int n = n0 + nn, k = k0 + kk;
-      Bs[kk][nn] = (n < Ncol && k < K) ? op.b(z, k, n) : make_double2(0.0, 0.0);
+      double2 v = (n < Ncol && k < K) ? op.b(z, k, n) : make_double2(0.0, 0.0);
+      if (MODE == kAbs1 || MODE == kAbs2) v = make_double2(hypot(v.x, v.y), 0.0);  // moduli once per element
+      Bs[kk][nn] = v;
     }
     __syncthreads();
 #pragma unroll 4
     for (int kk = 0; kk < BK; ++kk) {
       AT av[2];
-      double2 bv[4];
+      double2 bv[QN];
 #pragma unroll
       for (int r = 0; r < 2; ++r) av[r] = As[kk][tx + 16 * r];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) bv[q] = Bs[kk][ty + 16 * q];
+      for (int q = 0; q < QN; ++q) bv[q] = Bs[kk][ty + 16 * q];
 #pragma unroll
       for (int r = 0; r < 2; ++r)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < QN; ++q) {
           if constexpr (MODE == kComp1) {
             sr[r][q].add_prod(-av[r], bv[q].x);
             si[r][q].add_prod(-av[r], bv[q].y);
@@ -392,9 +404,9 @@ __global__ void __launch_bounds__(256) resid_tile2_kernel(Op op_all, int M, int 
             si[r][q].add_prod(-av[r].x, bv[q].y);
             si[r][q].add_prod(-av[r].y, bv[q].x);
           } else if constexpr (MODE == kAbs1) {
-            ar[r][q] = fma(fabs(av[r]), hypot(bv[q].x, bv[q].y), ar[r][q]);
+            ar[r][q] = fma(fabs(av[r]), bv[q].x, ar[r][q]);
           } else {
-            ar[r][q] = fma(hypot(av[r].x, av[r].y), hypot(bv[q].x, bv[q].y), ar[r][q]);
+            ar[r][q] = fma(av[r].x, bv[q].x, ar[r][q]);
           }
         }
     }
@@ -403,7 +415,7 @@ __global__ void __launch_bounds__(256) resid_tile2_kernel(Op op_all, int M, int 
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < QN; ++q) {
       const int m = m0 + tx + 16 * r, n = n0 + ty + 16 * q;
       if (m < M && n < Ncol) {
         const size_t idx = op.o(z, m, n, ldo);

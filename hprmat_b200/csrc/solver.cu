@@ -1268,48 +1268,60 @@ struct Operator {
   int nr = 0;
 };
 
+// Tiled products of the structured operator: plain (kinetic then coupling), and the outer-step
+// modes for `units` operators (resid_tile2_kernel), BN columns per tile.
+template <int BN>
+static int resid_plain(hprmat_b200_ctx* c, const KineticTile& kt, const CouplingTile& ct, int nr, int nch, int ncol,
+                       double2* out, long ldo) {
+  resid_tile_kernel<KineticTile, true, BN>
+      <<<dim3(cdiv_u(nr, 64), cdiv_u(ncol, BN), nch), 256, 0, c->stream>>>(kt, nr, ncol, nr, out, ldo);
+  LAUNCH_CHECK();
+  resid_tile_kernel<CouplingTile, false, BN>
+      <<<dim3(cdiv_u(nch, 64), cdiv_u(ncol, BN), nr), 256, 0, c->stream>>>(ct, nch, ncol, nch, out, ldo);
+  LAUNCH_CHECK();
+  return HPRMAT_B200_OK;
+}
+template <int BN, int M1, int M2>
+static int resid_outer(hprmat_b200_ctx* c, const KineticTile& kt, const CouplingTile& ct, int nr, int nch, int ncol,
+                       double2* out, long ldo, double2* lo, int units, long so) {
+  const int yt = (int)cdiv_u(ncol, BN);
+  const dim3 gk(cdiv_u(nr, 32), yt * units, nch), gc(cdiv_u(nch, 32), yt * units, nr);
+  resid_tile2_kernel<KineticTile, true, M1, BN><<<gk, 256, 0, c->stream>>>(kt, nr, ncol, nr, out, ldo, lo, yt, so);
+  LAUNCH_CHECK();
+  resid_tile2_kernel<CouplingTile, false, M2, BN>
+      <<<gc, 256, 0, c->stream>>>(ct, nch, ncol, nch, out, ldo, lo, yt, so);
+  LAUNCH_CHECK();
+  return HPRMAT_B200_OK;
+}
+template <int M1, int M2>
+static int resid_outer_any(hprmat_b200_ctx* c, const KineticTile& kt, const CouplingTile& ct, int nr, int nch, int ncol,
+                           double2* out, long ldo, double2* lo, int units, long so) {
+  switch (resid_bn(ncol)) {
+    case 16: return resid_outer<16, M1, M2>(c, kt, ct, nr, nch, ncol, out, ldo, lo, units, so);
+    case 32: return resid_outer<32, M1, M2>(c, kt, ct, nr, nch, ncol, out, ldo, lo, units, so);
+  }
+  return resid_outer<64, M1, M2>(c, kt, ct, nr, nch, ncol, out, ldo, lo, units, so);
+}
+
 // absmode: out = |B| + |C| |X| instead (structured operator only).
 static int apply_residual(hprmat_b200_ctx* c, const Operator& op, const double2* X, long ldx, int ncol,
                           double2* out, long ldo, bool with_b, bool absmode = false) {
   const int N = op.N;
-  if (op.structured && !with_b && !absmode) {
-    // plain product (inner iterations): tiled batched kernels
-    const int nr = op.mesh.nr;
-    KineticTile kt{op.mesh, op.ch, X, ldx, with_b ? 1 : 0};
-    resid_tile_kernel<KineticTile, true>
-        <<<dim3(cdiv_u(nr, 64), cdiv_u(ncol, 64), op.nch), 256, 0, c->stream>>>(kt, nr, ncol, nr, out, ldo);
-    LAUNCH_CHECK();
-    CouplingTile ct{op.vt, X, ldx, nr, op.nch};
-    resid_tile_kernel<CouplingTile, false>
-        <<<dim3(cdiv_u(op.nch, 64), cdiv_u(ncol, 64), nr), 256, 0, c->stream>>>(ct, op.nch, ncol, op.nch, out, ldo);
-    LAUNCH_CHECK();
-    return HPRMAT_B200_OK;
-  }
   if (op.structured) {
-    // outer residual (compensated, low words in rlo) or its rounding scale (absmode)
     const int nr = op.mesh.nr;
-    double2* lo = nullptr;
-    if (!absmode) {
-      TRY(c->rlo.ensure((size_t)ldo * ncol * sizeof(double2)));
-      lo = c->rlo.as<double2>();
+    const KineticTile kt{op.mesh, op.ch, X, ldx, with_b ? 1 : 0};
+    const CouplingTile ct{op.vt, X, ldx, nr, op.nch};
+    if (!with_b && !absmode) {  // plain product (inner iterations)
+      switch (resid_bn(ncol)) {
+        case 16: return resid_plain<16>(c, kt, ct, nr, op.nch, ncol, out, ldo);
+        case 32: return resid_plain<32>(c, kt, ct, nr, op.nch, ncol, out, ldo);
+      }
+      return resid_plain<64>(c, kt, ct, nr, op.nch, ncol, out, ldo);
     }
-    KineticTile kt{op.mesh, op.ch, X, ldx, with_b ? 1 : 0};
-    CouplingTile ct{op.vt, X, ldx, nr, op.nch};
-    const int yt = (int)cdiv_u(ncol, 64);
-    const dim3 gk(cdiv_u(nr, 32), yt, op.nch), gc(cdiv_u(op.nch, 32), yt, nr);
-    if (absmode) {
-      resid_tile2_kernel<KineticTile, true, kAbs1><<<gk, 256, 0, c->stream>>>(kt, nr, ncol, nr, out, ldo, lo, yt, 0);
-      LAUNCH_CHECK();
-      resid_tile2_kernel<CouplingTile, false, kAbs2><<<gc, 256, 0, c->stream>>>(ct, op.nch, ncol, op.nch, out, ldo,
-                                                                               lo, yt, 0);
-    } else {
-      resid_tile2_kernel<KineticTile, true, kComp1><<<gk, 256, 0, c->stream>>>(kt, nr, ncol, nr, out, ldo, lo, yt, 0);
-      LAUNCH_CHECK();
-      resid_tile2_kernel<CouplingTile, false, kComp2><<<gc, 256, 0, c->stream>>>(ct, op.nch, ncol, op.nch, out,
-                                                                                ldo, lo, yt, 0);
-    }
-    LAUNCH_CHECK();
-    return HPRMAT_B200_OK;
+    // outer residual (compensated, low words in rlo) or its rounding scale (absmode)
+    if (absmode) return resid_outer_any<kAbs1, kAbs2>(c, kt, ct, nr, op.nch, ncol, out, ldo, nullptr, 1, 0);
+    TRY(c->rlo.ensure((size_t)ldo * ncol * sizeof(double2)));
+    return resid_outer_any<kComp1, kComp2>(c, kt, ct, nr, op.nch, ncol, out, ldo, c->rlo.as<double2>(), 1, 0);
   }
   {
     dim3 g0(cdiv_u(N, 256), ncol);
@@ -1339,14 +1351,7 @@ static int apply_residual_units(hprmat_b200_ctx* c, const Operator& op, const do
   kt.sch = sch;
   CouplingTile ct{op.vt, X, ldx, nr, op.nch};
   ct.sx = sx;
-  const int yt = (int)cdiv_u(ncol, 64);
-  const dim3 gk(cdiv_u(nr, 32), yt * units, op.nch), gc(cdiv_u(op.nch, 32), yt * units, nr);
-  resid_tile2_kernel<KineticTile, true, kComp1><<<gk, 256, 0, c->stream>>>(kt, nr, ncol, nr, out, ldo, lo, yt, so);
-  LAUNCH_CHECK();
-  resid_tile2_kernel<CouplingTile, false, kComp2><<<gc, 256, 0, c->stream>>>(ct, op.nch, ncol, op.nch, out, ldo, lo,
-                                                                            yt, so);
-  LAUNCH_CHECK();
-  return HPRMAT_B200_OK;
+  return resid_outer_any<kComp1, kComp2>(c, kt, ct, nr, op.nch, ncol, out, ldo, lo, units, so);
 }
 
 static int frob_norm(hprmat_b200_ctx* c, const double2* X, long ldx, int N, int ncol, double* result) {
