@@ -182,15 +182,20 @@ __global__ void surface_rhs_kernel(MeshDev mesh, T* X, long ldx, int N, double s
 // FP64-bound: BN = 16, 32 or 64 by the columns at hand (resid_bn), since 8 right-hand sides in a
 // 64-wide tile were 7/8 padding (N = 400: compensated kinetic 29 -> 13 us, plain 17 -> 14 us,
 // moduli, now formed once per element, 28 -> 8 us; N = 6400, 32 columns: 165 -> 94, 59 -> 46 us).
-struct KineticTile {
+__device__ __forceinline__ double2 as_double2(double2 v) { return v; }
+__device__ __forceinline__ double2 as_double2(float2 v) { return make_double2((double)v.x, (double)v.y); }
+
+// XT: double2, or float2 (the FP32 solves' results, exact in FP64).
+template <typename XT>
+struct KineticTileOf {
   MeshDev mesh;
   ChannelData ch;
-  const double2* X;
+  const XT* X;
   long ldx;
   int with_b;
   long sx = 0, sch = 0;  // per-unit strides of X and of the channel data (batched launches)
-  __device__ KineticTile at(int u) const {
-    KineticTile t = *this;
+  __device__ KineticTileOf at(int u) const {
+    KineticTileOf t = *this;
     t.X += (size_t)u * sx;
     t.ch.fac += (size_t)u * sch;
     t.ch.kk += (size_t)u * sch;
@@ -206,29 +211,35 @@ struct KineticTile {
     }
     return k;
   }
-  __device__ double2 b(int c, int j, int col) const { return X[(size_t)c * mesh.nr + j + (size_t)col * ldx]; }
+  __device__ double2 b(int c, int j, int col) const {
+    return as_double2(X[(size_t)c * mesh.nr + j + (size_t)col * ldx]);
+  }
   __device__ size_t o(int c, int i, int col, long ldo) const { return (size_t)c * mesh.nr + i + (size_t)col * ldo; }
   __device__ double2 init(int c, int i, int col, const double2*, size_t) const {
     return make_double2(with_b ? surface_value(mesh, c, i, col) : 0.0, 0.0);
   }
 };
 
-struct CouplingTile {
+using KineticTile = KineticTileOf<double2>;
+
+template <typename XT>
+struct CouplingTileOf {
   const double2* vt;  // cpot_transpose_kernel layout
-  const double2* X;
+  const XT* X;
   long ldx;
   int nr, nch;
   long sx = 0;  // per-unit stride of X (batched launches)
-  __device__ CouplingTile at(int u) const {
-    CouplingTile t = *this;
+  __device__ CouplingTileOf at(int u) const {
+    CouplingTileOf t = *this;
     t.X += (size_t)u * sx;
     return t;
   }
   __device__ double2 a(int i, int c, int cp) const { return vt[((size_t)i * nch + cp) * nch + c]; }
-  __device__ double2 b(int i, int cp, int col) const { return X[(size_t)cp * nr + i + (size_t)col * ldx]; }
+  __device__ double2 b(int i, int cp, int col) const { return as_double2(X[(size_t)cp * nr + i + (size_t)col * ldx]); }
   __device__ size_t o(int i, int c, int col, long ldo) const { return (size_t)c * nr + i + (size_t)col * ldo; }
   __device__ double2 init(int, int, int, const double2* out, size_t idx) const { return out[idx]; }
 };
+using CouplingTile = CouplingTileOf<double2>;
 
 inline int resid_bn(int ncol) {
   if (ncol <= 16) return 16;
@@ -565,17 +576,6 @@ __global__ void d2f_matrix_kernel(const double2* __restrict__ src, long lds, flo
 // g[m+1] (complex).
 constexpr int kGmresMaxM = 16;  // longest FGMRES cycle
 
-// Per column |g_{j+1}| / beta: the cycle's residual reduction so far (for the host's
-// stopping test).  One thread per column.
-__global__ void gmres_estimate_kernel(const double2* __restrict__ g, const double* __restrict__ beta, int m, int j,
-                                      int ncol, double* out) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncol) return;
-  double2 v = g[(size_t)col * (m + 1) + j + 1];
-  double b = beta[col];
-  out[col] = b > 0 ? hypot(v.x, v.y) / b : 0.0;
-}
-
 struct GmresState {
   double2* V;     // [(m+1)][ldv * ncol]
   long ldv;
@@ -585,6 +585,8 @@ struct GmresState {
   double2* sn;    // [ncol][m]
   double2* g;     // [ncol][m+1]
   double* beta;   // [ncol] initial residual norm of each column
+  float2* Z;      // [m][ldv * ncol] V_j rounded to FP32, which the preconditioner turns into Z_j
+  double* est;    // [ncol] (host memory) |g_{j+1}| / beta: the cycle's residual reduction so far
   int m, N, ncol;
 };
 
@@ -609,7 +611,7 @@ __device__ inline double2 block_sum2(double2 v, double2* red) {
   return red[32];
 }
 
-// V_0 = r / |r|, g = (|r|, 0, ...).  r is V block 0 on entry.
+// V_0 = r / |r| (and its FP32 copy, Z block 0), g = (|r|, 0, ...).  r is V block 0 on entry.
 template <int NT>
 __global__ void __launch_bounds__(NT) gmres_start_kernel(GmresState s) {
   __shared__ double2 red[33];
@@ -622,9 +624,12 @@ __global__ void __launch_bounds__(NT) gmres_start_kernel(GmresState s) {
   }
   double beta = sqrt(block_sum2<NT>(acc, red).x);
   double inv = beta > 0 ? 1.0 / beta : 0.0;
+  float2* z = s.Z + (size_t)col * s.ldv;
   for (int r = threadIdx.x; r < s.N; r += NT) {
     double2 x = v[r];
-    v[r] = make_double2(x.x * inv, x.y * inv);
+    x = make_double2(x.x * inv, x.y * inv);
+    v[r] = x;
+    z[r] = to_f(x);
   }
   for (int i = threadIdx.x; i <= s.m; i += NT) s.g[(size_t)col * (s.m + 1) + i] = make_double2(i == 0 ? beta : 0.0, 0.0);
   if (threadIdx.x == 0) s.beta[col] = beta;
@@ -716,9 +721,12 @@ __global__ void __launch_bounds__(NT) gmres_arnoldi_kernel(GmresState s, int j) 
   double hn = sqrt(block_sum2<NT>(acc, red).x);
   const bool breakdown = !(hn > 1e-300);
   double inv = breakdown ? 0.0 : 1.0 / hn;
+  float2* z = j + 1 < m ? s.Z + (size_t)(j + 1) * s.vstride + (size_t)col * s.ldv : nullptr;
   for (int r = threadIdx.x; r < s.N; r += NT) {
     double2 b = w[r];
-    w[r] = make_double2(b.x * inv, b.y * inv);
+    b = make_double2(b.x * inv, b.y * inv);
+    w[r] = b;
+    if (z) z[r] = to_f(b);
   }
   if (threadIdx.x == 0) {
     double2* H = s.H + (size_t)col * (m + 1) * m;
@@ -765,14 +773,15 @@ __global__ void __launch_bounds__(NT) gmres_arnoldi_kernel(GmresState s, int j) 
     g[j] = make_double2(c * gj.x, c * gj.y);
     g[j + 1] = make_double2(-(sv.x * gj.x + sv.y * gj.y), -(sv.x * gj.y - sv.y * gj.x));
     for (int i = 0; i <= j + 1; ++i) H[(size_t)j * (m + 1) + i] = hc[i];
+    const double bt = s.beta[col];
+    s.est[col] = bt > 0 ? hypot(g[j + 1].x, g[j + 1].y) / bt : 0.0;
   }
 }
 
 // Solve the rotated (upper triangular) least-squares system for y and apply
 // X += sum_i y_i Z_i (flexible GMRES: Z_i = M^-1 V_i).  One CTA per column.
 template <int NT>
-__global__ void __launch_bounds__(NT) gmres_update_kernel(GmresState s, int jdone, const double2* Z, long zstride,
-                                                          long ldz, double2* X, long ldx, double sign) {
+__global__ void __launch_bounds__(NT) gmres_update_kernel(GmresState s, int jdone, double2* X, long ldx, double sign) {
   __shared__ double2 y[kGmresMaxM];
   const int col = blockIdx.x;
   const int m = s.m;
@@ -800,7 +809,7 @@ __global__ void __launch_bounds__(NT) gmres_update_kernel(GmresState s, int jdon
   for (int r = threadIdx.x; r < s.N; r += NT) {
     double2 acc = x[r];
     for (int i = 0; i < jdone; ++i) {
-      double2 z = Z[(size_t)i * zstride + (size_t)col * ldz + r];
+      const double2 z = to_d(s.Z[(size_t)i * s.vstride + (size_t)col * s.ldv + r]);
       acc.x += sign * (y[i].x * z.x - y[i].y * z.y);
       acc.y += sign * (y[i].x * z.y + y[i].y * z.x);
     }

@@ -146,7 +146,7 @@ struct hprmat_b200_ctx {
   DevBuf mesh;  // tc | blo0 | r | q2 | q1, each ns intervals, then the weights wle (nr)
   // work buffers
   DevBuf W, A64, X, X64, R64, B64, V, Z, gm, swaps, ipiv, stage, status, ops, inv, chan, rmat,
-      zwork, cpot, cu, norms, lup, rop, rsurf, vt, rlo, linv;
+      zwork, cpot, cu, lup, rop, rsurf, vt, rlo, linv;
   // wave functions: per-interval solutions and propagation matrices, surface amplitudes, cf
   DevBuf wfx, wfz, wfc, wfcf;
   DevBuf fpbuf;  // potential fingerprint (opts.reuse_factors)
@@ -215,7 +215,8 @@ struct hprmat_b200_ctx {
   std::vector<ScanTune> scan_tune;  // autotuner table, applied per unit by rmatrix_scan
   int wtrace_units = 0;
   int* h_status = nullptr;  // pinned
-  double* h_norms = nullptr;  // pinned
+  double* h_norms = nullptr;  // pinned; the norm kernels write it directly
+  size_t h_norms_n = 0;
   TcGemmPlan tcplan;
   // counters for benchmarks: kernel launches issued, and (when profiling) CUDA-event
   // time and algorithmic flops of the tensor-core trailing updates
@@ -1075,6 +1076,8 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     }
   }
   HPR_CUDA_TRY(cudaMemcpyAsync(c->h_status, status, kStatusCopy * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  if (mixed && tc_gemm_check_async(c->tcplan, c->stream))
+    return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
   HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (c->h_status[SW_TIMEOUT] != 0)
     return fail(HPRMAT_B200_ERR_TIMEOUT, "panel factorisation: grid barrier wait limit exceeded (site %d)",
@@ -1092,7 +1095,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   }
   if (mixed) {
     int err = 0;
-    TRY(tc_gemm_check(c->tcplan, c->stream, &err));
+    TRY(tc_gemm_check_done(c->tcplan, c->stream, &err));
     if (err) return fail(HPRMAT_B200_ERR_TIMEOUT, "tensor-core update: wait limit exceeded at site %d", err);
   }
   return HPRMAT_B200_OK;
@@ -1270,13 +1273,13 @@ struct Operator {
 
 // Tiled products of the structured operator: plain (kinetic then coupling), and the outer-step
 // modes for `units` operators (resid_tile2_kernel), BN columns per tile.
-template <int BN>
-static int resid_plain(hprmat_b200_ctx* c, const KineticTile& kt, const CouplingTile& ct, int nr, int nch, int ncol,
-                       double2* out, long ldo) {
-  resid_tile_kernel<KineticTile, true, BN>
+template <int BN, class KT, class CT>
+static int resid_plain(hprmat_b200_ctx* c, const KT& kt, const CT& ct, int nr, int nch, int ncol, double2* out,
+                       long ldo) {
+  resid_tile_kernel<KT, true, BN>
       <<<dim3(cdiv_u(nr, 64), cdiv_u(ncol, BN), nch), 256, 0, c->stream>>>(kt, nr, ncol, nr, out, ldo);
   LAUNCH_CHECK();
-  resid_tile_kernel<CouplingTile, false, BN>
+  resid_tile_kernel<CT, false, BN>
       <<<dim3(cdiv_u(nch, 64), cdiv_u(ncol, BN), nr), 256, 0, c->stream>>>(ct, nch, ncol, nch, out, ldo);
   LAUNCH_CHECK();
   return HPRMAT_B200_OK;
@@ -1303,6 +1306,20 @@ static int resid_outer_any(hprmat_b200_ctx* c, const KineticTile& kt, const Coup
   return resid_outer<64, M1, M2>(c, kt, ct, nr, nch, ncol, out, ldo, lo, units, so);
 }
 
+// out = -C X of the structured operator, X in FP32 or FP64 (inner iterations).
+template <typename XT>
+static int apply_product(hprmat_b200_ctx* c, const Operator& op, const XT* X, long ldx, int ncol, double2* out,
+                         long ldo) {
+  const int nr = op.mesh.nr;
+  const KineticTileOf<XT> kt{op.mesh, op.ch, X, ldx, 0};
+  const CouplingTileOf<XT> ct{op.vt, X, ldx, nr, op.nch};
+  switch (resid_bn(ncol)) {
+    case 16: return resid_plain<16>(c, kt, ct, nr, op.nch, ncol, out, ldo);
+    case 32: return resid_plain<32>(c, kt, ct, nr, op.nch, ncol, out, ldo);
+  }
+  return resid_plain<64>(c, kt, ct, nr, op.nch, ncol, out, ldo);
+}
+
 // absmode: out = |B| + |C| |X| instead (structured operator only).
 static int apply_residual(hprmat_b200_ctx* c, const Operator& op, const double2* X, long ldx, int ncol,
                           double2* out, long ldo, bool with_b, bool absmode = false) {
@@ -1311,13 +1328,7 @@ static int apply_residual(hprmat_b200_ctx* c, const Operator& op, const double2*
     const int nr = op.mesh.nr;
     const KineticTile kt{op.mesh, op.ch, X, ldx, with_b ? 1 : 0};
     const CouplingTile ct{op.vt, X, ldx, nr, op.nch};
-    if (!with_b && !absmode) {  // plain product (inner iterations)
-      switch (resid_bn(ncol)) {
-        case 16: return resid_plain<16>(c, kt, ct, nr, op.nch, ncol, out, ldo);
-        case 32: return resid_plain<32>(c, kt, ct, nr, op.nch, ncol, out, ldo);
-      }
-      return resid_plain<64>(c, kt, ct, nr, op.nch, ncol, out, ldo);
-    }
+    if (!with_b && !absmode) return apply_product(c, op, X, ldx, ncol, out, ldo);
     // outer residual (compensated, low words in rlo) or its rounding scale (absmode)
     if (absmode) return resid_outer_any<kAbs1, kAbs2>(c, kt, ct, nr, op.nch, ncol, out, ldo, nullptr, 1, 0);
     TRY(c->rlo.ensure((size_t)ldo * ncol * sizeof(double2)));
@@ -1354,12 +1365,21 @@ static int apply_residual_units(hprmat_b200_ctx* c, const Operator& op, const do
   return resid_outer_any<kComp1, kComp2>(c, kt, ct, nr, op.nch, ncol, out, ldo, lo, units, so);
 }
 
+// At least n doubles of pinned host memory that kernels write (c->h_norms); what was there is lost.
+static int norms_ensure(hprmat_b200_ctx* c, size_t n) {
+  if (n <= c->h_norms_n) return HPRMAT_B200_OK;
+  if (c->h_norms) cudaFreeHost(c->h_norms);
+  c->h_norms = nullptr;
+  c->h_norms_n = 0;
+  HPR_CUDA_TRY(cudaMallocHost(&c->h_norms, n * sizeof(double)));
+  c->h_norms_n = n;
+  return HPRMAT_B200_OK;
+}
+
 static int frob_norm(hprmat_b200_ctx* c, const double2* X, long ldx, int N, int ncol, double* result) {
-  TRY(c->norms.ensure((size_t)ncol * sizeof(double)));
-  colnorm2_kernel<<<ncol, 256, 0, c->stream>>>(X, ldx, N, c->norms.as<double>());
+  TRY(norms_ensure(c, ncol));
+  colnorm2_kernel<<<ncol, 256, 0, c->stream>>>(X, ldx, N, c->h_norms);
   LAUNCH_CHECK();
-  HPR_CUDA_TRY(cudaMemcpyAsync(c->h_norms, c->norms.p, (size_t)ncol * sizeof(double), cudaMemcpyDeviceToHost,
-                               c->stream));
   HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
   double s = 0.0;
   for (int i = 0; i < ncol; ++i) s += c->h_norms[i];
@@ -1383,15 +1403,17 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
   const long ldv = st.ld;
   const long vstride = ldv * nrhs;
   TRY(c->V.ensure((size_t)(m + 1) * vstride * sizeof(double2)));
-  TRY(c->Z.ensure((size_t)m * vstride * sizeof(double2)));
+  TRY(c->Z.ensure((size_t)m * vstride * sizeof(float2)));
+  if (!op.structured) TRY(c->R64.ensure((size_t)vstride * sizeof(double2)));
   TRY(c->gm.ensure((size_t)nrhs * ((m + 1) * m * sizeof(double2) + m * sizeof(double) + m * sizeof(double2) +
                                    (m + 1) * sizeof(double2) + 2 * sizeof(double)) + 256));
   TRY(c->X.ensure((size_t)ldv * nrhs * sizeof(float2)));
   double2* V = c->V.as<double2>();
-  double2* Z = c->Z.as<double2>();
+  float2* Z = c->Z.as<float2>();
   float2* X32 = c->X.as<float2>();
   GmresState gs;
   gs.V = V;
+  gs.Z = Z;
   gs.ldv = ldv;
   gs.vstride = vstride;
   unsigned char* gp = c->gm.as<unsigned char>();
@@ -1405,7 +1427,15 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
   gp += (size_t)nrhs * m * sizeof(double);
   gs.beta = reinterpret_cast<double*>(gp);
   gp += (size_t)nrhs * sizeof(double);
-  double* d_est = reinterpret_cast<double*>(gp);
+  // host values: |r|^2 and the rounding scale per column, R's change, the cycle's estimates
+  TRY(norms_ensure(c, 3 * (size_t)nrhs + 2));
+  double *h_res = c->h_norms, *h_scale = h_res + nrhs, *h_change = h_scale + nrhs, *h_est = h_change + 2;
+  gs.est = h_est;
+  auto norm_of = [&](const double* v) {
+    double t = 0.0;
+    for (int q = 0; q < nrhs; ++q) t += v[q];
+    return sqrt(t);
+  };
   gs.m = m;
   gs.N = N;
   gs.ncol = nrhs;
@@ -1422,12 +1452,10 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
   (void)cnorm;
   if (stats) stats->surface_change = -1.0;
   for (int outer = 0;; ++outer) {
+    // residual, R and the rounding scale, then one wait for all of them
     TRY(apply_residual(c, op, X64, ldx, nrhs, V, ldv, true));
-    double rn;
-    TRY(frob_norm(c, V, ldv, N, nrhs, &rn));
-    const double rel = rn / bnorm;
-    if (outer == 0) rel0 = rel;
-    double change = -1.0;
+    colnorm2_kernel<<<nrhs, 256, 0, c->stream>>>(V, ldv, N, h_res);
+    LAUNCH_CHECK();
     if (surf) {
       // R of the current iterate into slot (outer & 1); compare with the previous one
       double2* Rn = c->rsurf.as<double2>() + (size_t)(outer & 1) * nsurf;
@@ -1441,20 +1469,30 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
       }
       if (outer > 0) {
         const double2* Ro = c->rsurf.as<double2>() + (size_t)((outer - 1) & 1) * nsurf;
-        TRY(c->norms.ensure(2 * sizeof(double) * 2));
-        rel_change_kernel<<<1, 256, 0, c->stream>>>(Rn, Ro, (int)nsurf, c->norms.as<double>());
+        rel_change_kernel<<<1, 256, 0, c->stream>>>(Rn, Ro, (int)nsurf, h_change);
         LAUNCH_CHECK();
-        HPR_CUDA_TRY(cudaMemcpyAsync(c->h_norms, c->norms.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
-        change = c->h_norms[1] > 0 ? sqrt(c->h_norms[0] / c->h_norms[1]) : 0.0;
       }
     }
     if (op.structured && outer == 0) {
       // rounding scale of the residual: u || |B| + |C||X| ||_F / ||B||_F (reported only)
       TRY(apply_residual(c, op, X64, ldx, nrhs, V + vstride, ldv, true, true));
-      double fn;
-      TRY(frob_norm(c, V + vstride, ldv, N, nrhs, &fn));
-      floor_rel = 1.1102230246251565e-16 * fn / bnorm;
+      colnorm2_kernel<<<nrhs, 256, 0, c->stream>>>(V + vstride, ldv, N, h_scale);
+      LAUNCH_CHECK();
+    }
+    if (tc_gemm_check_async(c->tcplan, c->stream)) return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
+    HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    {
+      // a bounded wait that gave up inside a tensor-core solve invalidates the result
+      int err = 0;
+      TRY(tc_gemm_check_done(c->tcplan, c->stream, &err));
+      if (err) return fail(HPRMAT_B200_ERR_TIMEOUT, "tensor-core solve: wait limit exceeded at site %d", err);
+    }
+    const double rel = norm_of(h_res) / bnorm;
+    if (outer == 0) rel0 = rel;
+    double change = -1.0;
+    if (surf && outer > 0) change = h_change[1] > 0 ? sqrt(h_change[0] / h_change[1]) : 0.0;
+    if (op.structured && outer == 0) {
+      floor_rel = 1.1102230246251565e-16 * norm_of(h_scale) / bnorm;
       if (stats) stats->floor_history[0] = floor_rel;
     }
     if (stats && outer < 9) stats->residual_history[outer] = rel;
@@ -1514,30 +1552,30 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
     int jdone = 0;
     double est = 1.0;
     for (int j = 0; j < m; ++j) {
-      d2f_kernel<<<gconv, 256, 0, c->stream>>>(V + (size_t)j * vstride, ldv, X32, ldv, N, nullptr);
-      LAUNCH_CHECK();
-      TRY(lu_solve_tc(c, st, X32, ldv, nrhs));
-      f2d_kernel<<<gconv, 256, 0, c->stream>>>(X32, ldv, Z + (size_t)j * vstride, ldv, N, nullptr);
-      LAUNCH_CHECK();
+      // Z_j <- (LU)^-1 V_j in place on the FP32 copy of V_j that the step before left there
+      float2* Zj = Z + (size_t)j * vstride;
+      TRY(lu_solve_tc(c, st, Zj, ldv, nrhs));
       // V_{j+1} = -C Z_j: FGMRES runs on the operator -C, so the correction is subtracted
-      TRY(apply_residual(c, op, Z + (size_t)j * vstride, ldv, nrhs, V + (size_t)(j + 1) * vstride, ldv, false));
+      if (op.structured) {
+        TRY(apply_product(c, op, Zj, ldv, nrhs, V + (size_t)(j + 1) * vstride, ldv));
+      } else {
+        f2d_kernel<<<gconv, 256, 0, c->stream>>>(Zj, ldv, c->R64.as<double2>(), ldv, N, nullptr);
+        LAUNCH_CHECK();
+        TRY(apply_residual(c, op, c->R64.as<double2>(), ldv, nrhs, V + (size_t)(j + 1) * vstride, ldv, false));
+      }
       gmres_arnoldi_kernel<kArnoldiNT><<<nrhs, kArnoldiNT, 0, c->stream>>>(gs, j);
       LAUNCH_CHECK();
       jdone = j + 1;
       // residual estimate of the cycle (worst column) from the Givens-rotated right side
-      gmres_estimate_kernel<<<cdiv_u(nrhs, 128), 128, 0, c->stream>>>(gs.g, gs.beta, m, j, nrhs, d_est);
-      LAUNCH_CHECK();
-      HPR_CUDA_TRY(cudaMemcpyAsync(c->h_norms, d_est, (size_t)nrhs * sizeof(double), cudaMemcpyDeviceToHost,
-                                   c->stream));
       HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
       est = 0.0;
-      for (int q = 0; q < nrhs; ++q) est = std::max(est, c->h_norms[q]);
+      for (int q = 0; q < nrhs; ++q) est = std::max(est, h_est[q]);
       if (est < inner_tol) break;
     }
     last_est = est;
     prev_rel = rel;
     prev_change = change;
-    gmres_update_kernel<256><<<nrhs, 256, 0, c->stream>>>(gs, jdone, Z, vstride, ldv, X64, ldx, -1.0);
+    gmres_update_kernel<256><<<nrhs, 256, 0, c->stream>>>(gs, jdone, X64, ldx, -1.0);
     LAUNCH_CHECK();
     inner_total += jdone;
     ++steps;
@@ -1545,12 +1583,6 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
   if (stats) {
     stats->refine_steps = steps;
     stats->inner_iterations = inner_total;
-  }
-  {
-    // a bounded wait that gave up inside a tensor-core solve invalidates the result
-    int err = 0;
-    TRY(tc_gemm_check(c->tcplan, c->stream, &err));
-    if (err) return fail(HPRMAT_B200_ERR_TIMEOUT, "tensor-core solve: wait limit exceeded at site %d", err);
   }
   return status;
 }
@@ -2017,7 +2049,14 @@ static int rmatrix_core(hprmat_b200_ctx* c, int nch, const int* lval, const doub
                                             zo + std::max(1, no * no), d_cu, ndim, d_info);
   LAUNCH_CHECK();
   HPR_CUDA_TRY(cudaMemcpyAsync(c->h_status, c->status.p, SW_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  if (mixed && tc_gemm_check_async(c->tcplan, c->stream))
+    return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
   HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  if (mixed) {  // the refinement's last solve (after its own last check)
+    int err = 0;
+    TRY(tc_gemm_check_done(c->tcplan, c->stream, &err));
+    if (err) return fail(HPRMAT_B200_ERR_TIMEOUT, "tensor-core solve: wait limit exceeded at site %d", err);
+  }
   if (c->h_status[SW_INFO] != 0) return fail(HPRMAT_B200_SINGULAR, "singular Z_O in the collision-matrix step");
   if (wf) {
     // surface amplitudes from U, carried inwards, then the wave function per interval
@@ -2389,6 +2428,7 @@ int hprmat_b200_create(int device, const hprmat_b200_opts* opts, hprmat_b200_ctx
   c->own_stream = true;
   HPR_CUDA_TRY(cudaMallocHost(&c->h_status, 64 * sizeof(int)));
   HPR_CUDA_TRY(cudaMallocHost(&c->h_norms, 4096 * sizeof(double)));
+  c->h_norms_n = 4096;
   int s = c->status.ensure(64 * sizeof(int));
   if (s != HPRMAT_B200_OK) {
     delete c;
@@ -2410,7 +2450,7 @@ int hprmat_b200_destroy(hprmat_b200_ctx* c) {
   cudaStreamSynchronize(c->stream);
   DevBuf* bufs[] = {&c->mesh, &c->W, &c->A64, &c->X, &c->X64, &c->R64, &c->B64, &c->V, &c->Z, &c->gm,
                     &c->swaps, &c->ipiv, &c->stage, &c->status, &c->ops, &c->inv, &c->chan, &c->rmat,
-                    &c->zwork, &c->cpot, &c->cu, &c->norms, &c->lup, &c->rop, &c->rsurf, &c->vt, &c->rlo, &c->linv,
+                    &c->zwork, &c->cpot, &c->cu, &c->lup, &c->rop, &c->rsurf, &c->vt, &c->rlo, &c->linv,
                     &c->wfx, &c->wfz, &c->wfc, &c->wfcf, &c->fpbuf};
   for (DevBuf* b : bufs) b->release();
   for (hprmat_b200_ctx* w : c->scan_workers) hprmat_b200_destroy(w);
@@ -2419,6 +2459,8 @@ int hprmat_b200_destroy(hprmat_b200_ctx* c) {
   for (cudaEvent_t e : c->ev) cudaEventDestroy(e);
   if (c->h_status) cudaFreeHost(c->h_status);
   if (c->h_norms) cudaFreeHost(c->h_norms);
+  if (c->tcplan.h_err) cudaFreeHost(c->tcplan.h_err);
+  if (c->tcplan.d_err) cudaFree(c->tcplan.d_err);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return HPRMAT_B200_OK;

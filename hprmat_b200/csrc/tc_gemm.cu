@@ -277,6 +277,7 @@ int tc_gemm_init(TcGemmPlan& p, int device) {
   if (!p.d_err) {
     HPR_CUDA_TRY(cudaMalloc(&p.d_err, sizeof(int)));
     HPR_CUDA_TRY(cudaMemset(p.d_err, 0, sizeof(int)));
+    HPR_CUDA_TRY(cudaMallocHost(&p.h_err, sizeof(int)));
   }
   HPR_CUDA_TRY(cudaFuncSetAttribute(tc_update_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     TileCfg<256>::kSmemBytes));
@@ -335,13 +336,21 @@ int tc_update(TcGemmPlan& p, const TcOperand& A, int a_k0, int a_row0, const TcO
   return 0;
 }
 
-int tc_gemm_check(TcGemmPlan& p, cudaStream_t s, int* err_out) {
-  int h = 0;
-  HPR_CUDA_TRY(cudaMemcpyAsync(&h, p.d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  HPR_CUDA_TRY(cudaStreamSynchronize(s));
-  if (h) HPR_CUDA_TRY(cudaMemsetAsync(p.d_err, 0, sizeof(int), s));
-  *err_out = h;
+int tc_gemm_check_async(TcGemmPlan& p, cudaStream_t s) {
+  HPR_CUDA_TRY(cudaMemcpyAsync(p.h_err, p.d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
   return 0;
+}
+
+int tc_gemm_check_done(TcGemmPlan& p, cudaStream_t s, int* err_out) {
+  *err_out = *p.h_err;
+  if (*err_out) HPR_CUDA_TRY(cudaMemsetAsync(p.d_err, 0, sizeof(int), s));
+  return 0;
+}
+
+int tc_gemm_check(TcGemmPlan& p, cudaStream_t s, int* err_out) {
+  if (const int r = tc_gemm_check_async(p, s)) return r;
+  HPR_CUDA_TRY(cudaStreamSynchronize(s));
+  return tc_gemm_check_done(p, s, err_out);
 }
 
 }  // namespace hprmat

@@ -12,6 +12,7 @@ struct TcGemmPlan {
   int nsm = 0;
   void* encode = nullptr;  // cuTensorMapEncodeTiled, fetched through the runtime
   int* d_err = nullptr;    // device word: nonzero if a bounded wait gave up
+  int* h_err = nullptr;    // its pinned copy (tc_gemm_check_async)
   int max_grid = 0;        // most CTAs of a persistent update (0: one per SM); concurrent
                            // solves (scan workers) leave SMs to each other with a smaller grid
 };
@@ -37,5 +38,9 @@ int tc_update(TcGemmPlan& p, const TcOperand& A, int a_k0, int a_row0, const TcO
 
 // Reads and clears the device error word (0 = no wait gave up).
 int tc_gemm_check(TcGemmPlan& p, cudaStream_t s, int* err_out);
+// The same without a wait of its own: the copy is queued, and read after the caller's next
+// synchronisation of the stream.
+int tc_gemm_check_async(TcGemmPlan& p, cudaStream_t s);
+int tc_gemm_check_done(TcGemmPlan& p, cudaStream_t s, int* err_out);
 
 }  // namespace hprmat
