@@ -893,8 +893,9 @@ __device__ void cta_gauss_solve(double2* A, int n, double2* B, long ldb, int nrh
         if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
       }
       if (tid == 0) {
-        s_p = bi;
-        if (bv == 0.0 && *info == 0) *info = k + 1;
+        const bool none = bi >= n;  // every entry of the column is NaN: no pivot, and no row to exchange
+        s_p = none ? k : bi;
+        if ((none || bv == 0.0) && *info == 0) *info = k + 1;
       }
     }
     __syncthreads();
