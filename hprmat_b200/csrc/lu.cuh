@@ -11,8 +11,8 @@
 //                           and that row, then all CTAs pick the same pivot, swap and
 //                           eliminate their rows.  Writes ipiv and the step's row-interchange
 //                           list.
-//   2. trsm_lower_kernel -- applies the step's row interchanges to the columns right of the
-//                           panel (or to right-hand sides) and solves with the unit lower
+//   2. trsm_reg_kernel   -- applies the step's row interchanges to the columns right of the
+//      (trsm_lower_kernel)  panel (or to right-hand sides) and solves with the unit lower
 //                           diagonal block: U12 = L11^-1 P A12.
 //   3. trailing update   -- A22 -= L21 U12 (cgemm_update_kernel here; the mixed path uses
 //                           the tcgen05 kernel of tc_gemm.cu).
@@ -414,121 +414,182 @@ __global__ void __launch_bounds__(NT) trsm_lower_kernel(TrsmArgs<T> a) {
     for (int o = 16; o > 0; o >>= 1) gmax = fmax(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
     if ((tid & 31) == 0) atomicMax(a.growth_bits, mag_hi((double)gmax));
   }
-  if (a.lup != nullptr) {
-    for (int idx = tid; idx < ncw * ncols; idx += NT) {
-      int cc = idx % ncw, j = idx / ncw;
-      float hr, lr, hi_, li;
-      T v = A[cc * NBP + j];
-      tf32_split((float)v.x, hr, lr);
-      tf32_split((float)v.y, hi_, li);
-      size_t off = (size_t)(a.k0 + j) * a.lup_ld + (size_t)(cb + cc);
-      a.lup[off] = hr;
-      a.lup[a.lup_plane + off] = lr;
-      a.lup[2 * a.lup_plane + off] = hi_;
-      a.lup[3 * a.lup_plane + off] = li;
-    }
-  }
-  if (a.bop != nullptr) {
-    for (int idx = tid; idx < ncw * NB; idx += NT) {
-      int j = idx % NB, cc = idx / NB;
-      float hr = 0.f, lr = 0.f, hi_ = 0.f, li = 0.f;
-      if (j < ncols) {
-        T v = A[cc * NBP + j];
-        tf32_split((float)v.x, hr, lr);
-        tf32_split((float)v.y, hi_, li);
-      }
-      size_t off = (size_t)(cb + cc - a.bop_col0) * NB + j;
-      a.bop[0 * a.bop_plane + off] = hr;
-      a.bop[1 * a.bop_plane + off] = lr;
-      a.bop[2 * a.bop_plane + off] = hi_;
-      a.bop[3 * a.bop_plane + off] = li;
-    }
+}
+
+// trsm_lower_kernel with the right-hand sides in registers: LN = NB / 16 lanes share a column, lane g
+// holding rows LN a + g in x[a], a < 16.  A step broadcasts x_k within the lanes of a column and
+// updates the rows below; L11 is staged in shared memory once per CTA, and a group of 2 NB threads
+// walks over blocks of 32 columns (one barrier and one L2 read of L's column per step in
+// trsm_lower_kernel, no barrier here).  x moves one register down every LN steps and its end takes the
+// finished row, so that the code of LN steps serves several blocks of them and the rows are back in
+// place after 16; the displaced rows travel through the same shared memory meanwhile.  The operations
+// of trsm_lower_kernel in its order.
+// Measured, average over the steps: FP64, N = 4000 with NB = 64 41 -> 12 us.  Mixed, NB = 128, against
+// the inverse of L11, a row gather, a tensor-core product and a split of its result as four launches:
+// N = 400 40 -> 22 us, N = 3000 46 -> 23, N = 6400 48 -> 27, N = 25600 66 -> 71 (0.3 % of that
+// factorisation); and no inverse enters U any more.  Bound by the chain of NB broadcasts and updates,
+// in the wide case by the traffic of U12's three copies.
+// One group per CTA while the blocks do not fill the SMs, else two, which hide each other's latency
+// (N = 25600: 78 us with one, 71 with two, 87 with two columns per thread).
+constexpr int kTrsmCols = 32;
+template <int NB> constexpr int trsm_threads() { return kTrsmCols * (NB / 16); }  // of a group
+template <typename T, int NB> constexpr size_t trsm_smem(int groups) {
+  return ((size_t)NB * (NB + 1) + (size_t)groups * kTrsmCols * (NB + 1)) * sizeof(T);
+}
+
+template <typename T, int LN, int Q>
+__device__ __forceinline__ void trsm_block(T (&x)[16], const T* L, int ldl, int g) {
+  // LN steps: x[q] holds row LN q + g of the rows from this block on; L at its diagonal block.  The
+  // finished rows among the Q meet rows of L past the last one, that is the zeros above the diagonal
+  // of the next column.
+#pragma unroll
+  for (int e = 0; e < LN; ++e) {
+    T xk;
+    xk.x = LN > 1 ? __shfl_sync(0xffffffffu, x[0].x, e, LN) : x[0].x;
+    xk.y = LN > 1 ? __shfl_sync(0xffffffffu, x[0].y, e, LN) : x[0].y;
+    const T* Lc = L + (size_t)e * ldl + g;
+    if (g > e) cfms(x[0], Lc[0], xk);
+#pragma unroll
+    for (int q = 1; q < Q; ++q) cfms(x[q], Lc[LN * q], xk);
   }
 }
 
-// trsm_lower_kernel of the FP64 LU's block steps (NB = 64) with the right-hand sides in registers:
-// 4 lanes share a column, lane g holding rows 4 a + g in x[a].  A step broadcasts x_k within the
-// 4 lanes and updates the rows below; L11 is staged in shared memory once, and no block barrier
-// separates the steps (trsm_lower_kernel: one barrier and one L2 read of L's column per step, 41 us
-// for up to 4000 columns; here 17 us).  x moves one register down every 4 steps, so that the code of
-// 4 steps serves all 64.  The same operations in the same order as trsm_lower_kernel.
-constexpr int kTrsmCols = 32;  // columns per CTA of 128 threads
-constexpr int kTrsmNB = 64;
-constexpr int kTrsmLdL = kTrsmNB + 1;  // L11 by rows: the 4 lanes of a column read 4 rows of a column
-constexpr size_t kTrsmSmem = ((size_t)kTrsmNB * kTrsmLdL + 2 * (size_t)kTrsmCols * (kTrsmNB + 1)) * sizeof(double2);
-template <int NB>
-__global__ void __launch_bounds__(128) trsm_lower_f64_kernel(TrsmArgs<double2> a) {
-  constexpr int R = NB / 4, LDA = NB + 1;
+template <typename T, int NB>
+__global__ void __launch_bounds__(2 * trsm_threads<NB>()) trsm_reg_kernel(TrsmArgs<T> a) {
+  using R = typename RealOf<T>::R;
+  constexpr int LN = NB / 16, NT = trsm_threads<NB>(), LDA = NB + 1, CW = kTrsmCols;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* L = reinterpret_cast<double2*>(smem_raw);   // [i][k]
-  double2* A = L + (size_t)NB * kTrsmLdL;              // [column][row]
-  double2* E = A + (size_t)kTrsmCols * LDA;            // displaced rows
-  const int tid = threadIdx.x;
-  const int cb = a.c_begin + blockIdx.x * kTrsmCols;
-  const int ncw = min(kTrsmCols, a.c_end - cb);
-  if (ncw <= 0) return;
+  T* L = reinterpret_cast<T*>(smem_raw);  // column-major, strictly lower part, and one column of zeros
+  const int grp = threadIdx.x / NT, tid = threadIdx.x % NT, ngrp = (int)blockDim.x / NT;
+  T* A = L + (size_t)NB * (NB + 1) + (size_t)grp * CW * LDA;  // [column][row]
+  auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(NT) : "memory"); };
   const int ncols = a.ncols;
   const bool swap = a.mode != 2, solve = a.mode != 1;
   const int ne = swap ? *a.n_extra : 0;
-  if (solve)
-    for (int idx = tid; idx < NB * NB; idx += 128) {
-      const int i = idx % NB, k = idx / NB;
-      if (i < ncols && k < i) cp_async_elem(L + i * kTrsmLdL + k, a.W + (size_t)(a.k0 + i) + (size_t)(a.k0 + k) * a.ld);
-      else L[i * kTrsmLdL + k] = czero<double2>();
-    }
-  for (int idx = tid; idx < ncw * NB; idx += 128) {
-    const int j = idx % NB, cc = idx / NB;
-    if (j < ncols)
-      cp_async_elem(A + cc * LDA + j, a.X + (size_t)(swap ? a.top_src[j] : a.k0 + j) + (size_t)(cb + cc) * a.ldx);
-    else
-      A[cc * LDA + j] = czero<double2>();
-  }
-  for (int idx = tid; idx < ncw * ne; idx += 128) {
-    const int e = idx % ne, cc = idx / ne;
-    cp_async_elem(E + cc * LDA + e, a.X + (size_t)a.extra_src[e] + (size_t)(cb + cc) * a.ldx);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  for (int idx = tid; idx < ncw * ne; idx += 128) {
-    const int e = idx % ne, cc = idx / ne;
-    a.X[(size_t)a.extra_dst[e] + (size_t)(cb + cc) * a.ldx] = E[cc * LDA + e];
-  }
-  const int g = tid & 3, cc = tid >> 2;  // this thread's row class and column
-  double gmax = 0.0;
   if (solve) {
-    double2* col = A + (size_t)min(cc, ncw - 1) * LDA;
-    double2 x[R];
+    // 16-byte copies where the columns are aligned for them; zero outside the strictly lower part of
+    // ncols x ncols: trsm_block also reads there, for rows that are finished or do not exist
+    constexpr int V = 16 / (int)sizeof(T);
+    const T* Wl = a.W + (size_t)a.k0 + (size_t)a.k0 * a.ld;
+    const bool wide = a.ld % V == 0 && (reinterpret_cast<uintptr_t>(Wl) & 15) == 0;
+    for (int idx = threadIdx.x; idx < NB * (NB / V) + NB / V; idx += blockDim.x) {
+      const int k = idx / (NB / V), i = idx % (NB / V) * V;
+      T* d = L + (size_t)k * NB + i;
+      const T* src = Wl + i + (size_t)k * a.ld;
+      if (k < ncols && wide && i > k && i + V <= ncols) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src)
+                     : "memory");
+      } else {
 #pragma unroll
-    for (int q = 0; q < R; ++q) x[q] = col[4 * q + g];
-    for (int kb = 0; kb < R; ++kb) {  // x[q] holds row 4 (kb + q) + g
-      const double2* Lr = L + (size_t)(4 * kb + g) * kTrsmLdL + 4 * kb;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        // x_k, k = 4 kb + e, from lane e of the column
-        double2 xk;
-        xk.x = __shfl_sync(0xffffffffu, x[0].x, e, 4);
-        xk.y = __shfl_sync(0xffffffffu, x[0].y, e, 4);
-        if (g > e) cfms(x[0], Lr[e], xk);
-#pragma unroll
-        for (int q = 1; q < R; ++q)
-          if (kb + q < R) cfms(x[q], Lr[(size_t)4 * q * kTrsmLdL + e], xk);
+        for (int v = 0; v < V; ++v) {
+          if (k < ncols && i + v > k && i + v < ncols)
+            cp_async_elem(d + v, src + v);
+          else
+            d[v] = czero<T>();
+        }
       }
-      if (cc < ncw) col[4 * kb + g] = x[0];
-#pragma unroll
-      for (int q = 0; q + 1 < R; ++q) x[q] = x[q + 1];
     }
+    cp_async_wait_all();
     __syncthreads();
   }
-  for (int idx = tid; idx < ncw * NB; idx += 128) {
-    const int j = idx % NB, c = idx / NB;
-    if (j >= ncols) continue;
-    const double2 v = A[c * LDA + j];
-    a.X[(size_t)(a.k0 + j) + (size_t)(cb + c) * a.ldx] = v;
-    gmax = fmax(gmax, cabs1(v));
+  R gmax = R(0);
+  // copies: row j of every second column; the indexes stay out of the loops
+  static_assert(NT == 2 * NB, "two columns per pass");
+  const int j = tid % NB, c0 = tid / NB;
+  const bool has = j < ncols, ext = j < ne;
+  const size_t top = (size_t)(swap && has ? a.top_src[j] : a.k0 + j);
+  const size_t esrc = ext ? (size_t)a.extra_src[j] : 0, edst = ext ? (size_t)a.extra_dst[j] : 0;
+  for (int cb = a.c_begin + ((int)blockIdx.x * ngrp + grp) * CW; cb < a.c_end; cb += (int)gridDim.x * ngrp * CW) {
+    const int ncw = min(CW, a.c_end - cb);
+    T* Xc = a.X + (size_t)cb * a.ldx;
+    for (int cc = c0; cc < ncw; cc += 2) {
+      if (has)
+        cp_async_elem(A + cc * LDA + j, Xc + top + (size_t)cc * a.ldx);
+      else
+        A[cc * LDA + j] = czero<T>();
+    }
+    cp_async_wait_all();
+    group_sync();
+    const int g = tid % LN, cs = tid / LN;  // this thread's row class and column
+    T* col = A + min(cs, ncw - 1) * LDA + g;
+    T x[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) x[q] = col[LN * q];
+    group_sync();
+    if (ext)
+      for (int cc = c0; cc < ncw; cc += 2) cp_async_elem(A + cc * LDA + j, Xc + esrc + (size_t)cc * a.ldx);
+    if (solve) {
+      for (int kb = 0; kb < 16; ++kb) {
+        if (LN * kb < ncols) {
+          const T* Lb = L + (size_t)LN * kb * NB + LN * kb;
+          switch (kb >> 2) {
+            case 0: trsm_block<T, LN, 16>(x, Lb, NB, g); break;
+            case 1: trsm_block<T, LN, 12>(x, Lb, NB, g); break;
+            case 2: trsm_block<T, LN, 8>(x, Lb, NB, g); break;
+            default: trsm_block<T, LN, 4>(x, Lb, NB, g); break;
+          }
+        }
+        const T done = x[0];
+#pragma unroll
+        for (int q = 0; q + 1 < 16; ++q) x[q] = x[q + 1];
+        x[15] = done;
+      }
+    }
+    cp_async_wait_all();
+    group_sync();
+    if (ext)  // every row of X this block needs has been read
+      for (int cc = c0; cc < ncw; cc += 2) Xc[edst + (size_t)cc * a.ldx] = A[cc * LDA + j];
+    group_sync();
+    if (cs < ncw) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) col[LN * q] = x[q];
+    }
+    group_sync();
+    T* Xo = Xc + a.k0 + j;
+    if (has) {
+#pragma unroll 4
+      for (int cc = c0; cc < ncw; cc += 2) {
+        const T v = A[cc * LDA + j];
+        Xo[(size_t)cc * a.ldx] = v;
+        gmax = fmax(gmax, cabs1(v));
+      }
+    }
+    if (a.bop != nullptr) {  // B operand of the trailing update (zero beyond ncols)
+      float* b = a.bop + (size_t)(cb - a.bop_col0) * NB + j;
+#pragma unroll 4
+      for (int cc = c0; cc < ncw; cc += 2) {
+        const T v = A[cc * LDA + j];
+        float hr, lr, hi_, li;
+        tf32_split((float)v.x, hr, lr);
+        tf32_split((float)v.y, hi_, li);
+        b[(size_t)cc * NB] = hr;
+        b[(size_t)cc * NB + a.bop_plane] = lr;
+        b[(size_t)cc * NB + 2 * a.bop_plane] = hi_;
+        b[(size_t)cc * NB + 3 * a.bop_plane] = li;
+      }
+    }
+    if (a.lup != nullptr) {  // row-major: consecutive threads on consecutive columns
+      if (const int cc = tid % 32; cc < ncw) {
+        float* d = a.lup + (size_t)a.k0 * a.lup_ld + (size_t)(cb + cc);
+#pragma unroll 4
+        for (int jj = tid / 32; jj < ncols; jj += NT / 32) {
+          const T v = A[cc * LDA + jj];
+          float hr, lr, hi_, li;
+          tf32_split((float)v.x, hr, lr);
+          tf32_split((float)v.y, hi_, li);
+          float* e = d + (size_t)jj * a.lup_ld;
+          e[0] = hr;
+          e[a.lup_plane] = lr;
+          e[2 * a.lup_plane] = hi_;
+          e[3 * a.lup_plane] = li;
+        }
+      }
+    }
+    group_sync();
   }
   if (a.growth_bits && solve) {
     for (int o = 16; o > 0; o >>= 1) gmax = fmax(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
-    if ((tid & 31) == 0) atomicMax(a.growth_bits, mag_hi(gmax));
+    if ((tid & 31) == 0 && gmax > R(0)) atomicMax(a.growth_bits, mag_hi((double)gmax));
   }
 }
 
@@ -874,128 +935,6 @@ __global__ void __launch_bounds__(NB * CW) diag_apply_kernel(const T* __restrict
     rop[rop_plane + off] = lr;
     rop[2 * rop_plane + off] = hi_;
     rop[3 * rop_plane + off] = li;
-  }
-}
-
-// -------------------------------------------------------------------------------------
-// Tensor-core TRSM of the mixed path (U12 = L11^-1 P A12), in three steps per block step:
-//   l11_inverse_planes_kernel: Linv = L11^-1 (unit lower) written as the A-operand planes of (I - Linv), K-major rows;
-//   swap_gather_kernel: applies the step's row interchanges to the columns right of the
-//       panel, leaving P A12 in rows k0.. of W and as B-operand planes (per column K-major);
-//   tc_update: C -= (I - Linv) (P A12) with C = those rows of W, i.e. C = Linv P A12 = U12;
-//   u12_split_kernel: U12 -> B-operand planes of the trailing update and the LU planes.
-// One CTA per 16 columns of L11^-1 (tri_block_inverse); 38 us per step with the recursive joins of
-// the whole block on one SM before, 13 us now.
-template <int NB>
-__global__ void __launch_bounds__(256) l11_inverse_planes_kernel(const float2* __restrict__ W, long ld, int k0,
-                                                                 int ncols, float* planes, long plane) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int jb = blockIdx.x;
-  const float2* X = tri_block_inverse<float2, NB>(smem_raw, false, jb, W + (size_t)k0 + (size_t)k0 * ld, ld, ncols);
-  // (I - Linv) as A-operand planes: row i, K index j contiguous
-  for (int idx = threadIdx.x; idx < NB * kTiB; idx += 256) {
-    const int i = idx / kTiB, c = idx % kTiB, j = jb * kTiB + c;
-    const float2 v = X[(size_t)i * kTiLd + c];
-    float2 d = make_float2((i == j ? 1.f : 0.f) - v.x, -v.y);
-    if (i >= ncols || j >= ncols) d = make_float2(0.f, 0.f);
-    float hr, lr, hi_, li;
-    tf32_split(d.x, hr, lr);
-    tf32_split(d.y, hi_, li);
-    const size_t off = (size_t)i * NB + j;
-    planes[off] = hr;
-    planes[plane + off] = lr;
-    planes[2 * plane + off] = hi_;
-    planes[3 * plane + off] = li;
-  }
-}
-
-// Row interchanges of one step on columns [c_begin, c_end) of W, leaving P A12 in rows
-// k0 .. k0+ncols and as B-operand planes bg[(col - c_begin) * NB + j] (zero padded).
-template <int NB, int CW, int NT>
-__global__ void __launch_bounds__(NT) swap_gather_kernel(float2* W, long ld, int k0, int ncols,
-                                                         const int* __restrict__ top_src,
-                                                         const int* __restrict__ extra_dst,
-                                                         const int* __restrict__ extra_src,
-                                                         const int* __restrict__ n_extra, int c_begin, int c_end,
-                                                         float* bg, long plane) {
-  constexpr int NBP = NB + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* A = reinterpret_cast<float2*>(smem_raw);  // [CW][NBP]
-  float2* E = A + CW * NBP;                         // [CW][NB]
-  const int tid = threadIdx.x;
-  const int cb = c_begin + blockIdx.x * CW;
-  const int ncw = min(CW, c_end - cb);
-  if (ncw <= 0) return;
-  const int ne = *n_extra;
-  for (int idx = tid; idx < ncw * ncols; idx += NT) {
-    int j = idx % ncols, cc = idx / ncols;
-    A[cc * NBP + j] = W[(size_t)top_src[j] + (size_t)(cb + cc) * ld];
-  }
-  for (int idx = tid; idx < ncw * ne; idx += NT) {
-    int e = idx % ne, cc = idx / ne;
-    E[cc * NB + e] = W[(size_t)extra_src[e] + (size_t)(cb + cc) * ld];
-  }
-  __syncthreads();
-  for (int idx = tid; idx < ncw * ne; idx += NT) {
-    int e = idx % ne, cc = idx / ne;
-    W[(size_t)extra_dst[e] + (size_t)(cb + cc) * ld] = E[cc * NB + e];
-  }
-  for (int idx = tid; idx < ncw * NB; idx += NT) {
-    int j = idx % NB, cc = idx / NB;
-    float2 v = j < ncols ? A[cc * NBP + j] : make_float2(0.f, 0.f);
-    if (j < ncols) W[(size_t)(k0 + j) + (size_t)(cb + cc) * ld] = v;
-    float hr, lr, hi_, li;
-    tf32_split(v.x, hr, lr);
-    tf32_split(v.y, hi_, li);
-    size_t off = (size_t)(cb + cc - c_begin) * NB + j;
-    bg[off] = hr;
-    bg[plane + off] = lr;
-    bg[2 * plane + off] = hi_;
-    bg[3 * plane + off] = li;
-  }
-}
-
-// U12 (rows k0 .. k0+ncols of W, columns [c_begin, c_end)) -> B-operand planes of the
-// trailing update (per column K-major) and the row-major LU planes; tracks max |u_ij|.
-template <int NB, int CW, int NT>
-__global__ void __launch_bounds__(NT) u12_split_kernel(const float2* __restrict__ W, long ld, int k0, int ncols,
-                                                       int c_begin, int c_end, float* bop, long bplane, float* lup,
-                                                       long lup_ld, long lup_plane, unsigned* growth_bits) {
-  const int tid = threadIdx.x;
-  const int cb = c_begin + blockIdx.x * CW;
-  const int ncw = min(CW, c_end - cb);
-  if (ncw <= 0) return;
-  float gmax = 0.f;
-  // per column K-major operand: consecutive threads -> consecutive rows of one column
-  for (int idx = tid; idx < ncw * NB; idx += NT) {
-    int j = idx % NB, cc = idx / NB;
-    float2 v = j < ncols ? W[(size_t)(k0 + j) + (size_t)(cb + cc) * ld] : make_float2(0.f, 0.f);
-    gmax = fmaxf(gmax, fabsf(v.x) + fabsf(v.y));
-    float hr, lr, hi_, li;
-    tf32_split(v.x, hr, lr);
-    tf32_split(v.y, hi_, li);
-    size_t off = (size_t)(cb + cc - c_begin) * NB + j;
-    bop[off] = hr;
-    bop[bplane + off] = lr;
-    bop[2 * bplane + off] = hi_;
-    bop[3 * bplane + off] = li;
-  }
-  // row-major LU planes: consecutive threads -> consecutive columns of one row
-  for (int idx = tid; idx < ncw * ncols; idx += NT) {
-    int cc = idx % ncw, j = idx / ncw;
-    float2 v = W[(size_t)(k0 + j) + (size_t)(cb + cc) * ld];
-    float hr, lr, hi_, li;
-    tf32_split(v.x, hr, lr);
-    tf32_split(v.y, hi_, li);
-    size_t off = (size_t)(k0 + j) * lup_ld + (size_t)(cb + cc);
-    lup[off] = hr;
-    lup[lup_plane + off] = lr;
-    lup[2 * lup_plane + off] = hi_;
-    lup[3 * lup_plane + off] = li;
-  }
-  if (growth_bits) {
-    for (int o = 16; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
-    if ((tid & 31) == 0 && gmax > 0.f) atomicMax(growth_bits, mag_hi((double)gmax));
   }
 }
 

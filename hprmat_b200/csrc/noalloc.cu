@@ -140,9 +140,8 @@ extern "C" int hprmat_b200_solve_linear_noalloc(const void* d_A, void* d_B, int 
     void* args[] = {&pa};
     HPR_CUDA_TRY(cudaLaunchCooperativeKernel((void*)pk, dim3(G), dim3(NT), args, smem, st));
     if (k0 + ncols >= N) break;
-    constexpr int CW = 32;
-    auto tk = trsm_lower_kernel<T, NB, CW, NT>;
-    const size_t tsm = (size_t)CW * (NB + 1) * sizeof(T) + (size_t)CW * NB * sizeof(T);
+    auto tk = trsm_reg_kernel<T, NB>;
+    const size_t tsm = trsm_smem<T, NB>(1);
     if (tsm > 48 * 1024) HPR_CUDA_TRY(cudaFuncSetAttribute(tk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm));
     TrsmArgs<T> ta{};
     ta.W = W;
@@ -157,7 +156,7 @@ extern "C" int hprmat_b200_solve_linear_noalloc(const void* d_A, void* d_B, int 
     ta.ldx = ld;
     ta.c_begin = k0 + ncols;
     ta.c_end = N;
-    tk<<<(N - k0 - ncols + CW - 1) / CW, NT, tsm, st>>>(ta);
+    tk<<<(N - k0 - ncols + kTrsmCols - 1) / kTrsmCols, trsm_threads<NB>(), tsm, st>>>(ta);
     HPR_CUDA_TRY(cudaGetLastError());
     const int M2 = N - k0 - ncols;
     dim3 grid((M2 + 63) / 64, (M2 + 63) / 64);

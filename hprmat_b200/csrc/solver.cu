@@ -146,13 +146,13 @@ struct hprmat_b200_ctx {
   DevBuf mesh;  // tc | blo0 | r | q2 | q1, each ns intervals, then the weights wle (nr)
   // work buffers
   DevBuf W, A64, X, X64, R64, B64, V, Z, gm, swaps, ipiv, stage, status, ops, inv, chan, rmat,
-      zwork, cpot, cu, lup, rop, rsurf, vt, rlo, linv;
+      zwork, cpot, cu, lup, rop, rsurf, vt, rlo;
   // wave functions: per-interval solutions and propagation matrices, surface amplitudes, cf
   DevBuf wfx, wfz, wfc, wfcf;
   DevBuf fpbuf;  // potential fingerprint (opts.reuse_factors)
   DevBuf cond_v;  // condition estimate: one right-hand side (opts.estimate_condition)
   // tensor-core operand views of the current factorisation (mixed path)
-  TcOperand op_lu, op_bop, op_rhs, op_linv;
+  TcOperand op_lu, op_bop, op_rhs;
   long lup_ld = 0, lup_plane = 0, rop_plane = 0;
   int rop_nrhs = 0, rop_nb = 0;  // key of the solves' right-hand-side planes and their TMA map
   // wavefront solves (mixed path, nb = 128): sigma maps and permutation, transposed
@@ -166,7 +166,6 @@ struct hprmat_b200_ctx {
   bool wave_enabled = true;  // wavefront solves (else block-step solves)
   bool inv_ready = false;    // explicit inverses of the current factors (tri_solve.cuh)
   DevBuf invm, invy;         // L^-1 and U^-1; the product with L^-1
-  bool tc_trsm = true;       // U12 by the tensor cores from L11^-1 (else substitution)
   int panel_rpc_min = 32;    // fewest panel rows per CTA
   double growth_limit = 1e6;  // mixed path: pivot growth above which C(E) is factorised in FP64
   bool panel_cluster = true;  // panels that fit in one 16-CTA cluster use panel_reg_kernel
@@ -655,10 +654,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     c->lup_ld = (N + 3) / 4 * 4;
     c->lup_plane = c->lup_ld * (long)N;
     TRY(c->lup.ensure((size_t)4 * c->lup_plane * sizeof(float)));
-    TRY(c->linv.ensure((size_t)4 * NB * NB * sizeof(float)));
     if (N > NB) {  // views are used only when there is more than one block step
-      if (tc_make_operand(c->tcplan, c->op_linv, c->linv.as<float>(), NB, NB, NB, (long)NB * NB, 128))
-        return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
       if (tc_make_operand(c->tcplan, c->op_lu, c->lup.as<float>(), N, N, c->lup_ld, c->lup_plane, 128))
         return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
       if (tc_make_operand(c->tcplan, c->op_bop, bop, NB, N, NB, plane, 128))
@@ -684,15 +680,24 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     ta.c_end = c_end;
     ta.growth_bits = growth;
     ta.mode = mode;
-    if constexpr (std::is_same<T, double2>::value && NB == kTrsmNB) {
-      TRY(set_smem(trsm_lower_f64_kernel<NB>, kTrsmSmem));
-      trsm_lower_f64_kernel<NB><<<cdiv_u(c_end - c_begin, kTrsmCols), 128, kTrsmSmem, c->stream>>>(ta);
-    } else {
+    ta.bop = bop;  // mixed: U12 also as the B operand of the trailing update and into the LU planes
+    ta.bop_plane = plane;
+    ta.bop_col0 = c_begin;
+    ta.lup = mixed ? c->lup.as<float>() : nullptr;
+    ta.lup_ld = c->lup_ld;
+    ta.lup_plane = c->lup_plane;
+    if constexpr (sizeof(T) == sizeof(double2) && NB == 128) {  // L11 does not fit in shared memory
       constexpr int CW = 32;
       auto tk = trsm_lower_kernel<T, NB, CW, NT>;
       const size_t tsm = (size_t)CW * (NB + 1) * sizeof(T) + (size_t)CW * NB * sizeof(T);
       TRY(set_smem(tk, tsm));
       tk<<<cdiv_u(c_end - c_begin, CW), NT, tsm, c->stream>>>(ta);
+    } else {
+      auto tk = trsm_reg_kernel<T, NB>;
+      const unsigned blocks = cdiv_u(c_end - c_begin, kTrsmCols), ctas = (NB == 128 ? 1u : 2u) * (unsigned)c->nsm;
+      const int groups = NB == 128 && blocks > ctas ? 2 : 1;
+      TRY(set_smem(tk, trsm_smem<T, NB>(groups)));
+      tk<<<std::min(cdiv_u(blocks, groups), ctas), groups * trsm_threads<NB>(), trsm_smem<T, NB>(groups), c->stream>>>(ta);
     }
     LAUNCH_CHECK();
     return HPRMAT_B200_OK;
@@ -701,63 +706,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   auto after_panel = [&](int s, int k0, int ncols, const StepSwaps& sw) -> int {
     (void)s;
     // row interchanges + U12 = L11^-1 A12
-    if (mixed && c->tc_trsm) {
-      // L11^-1 (as I - L11^-1 operand planes), P A12 gathered, U12 by one tensor-core GEMM
-      constexpr int CW = 32;
-      const size_t ism = tri_block_smem<float2, NB>();
-      auto ik = l11_inverse_planes_kernel<NB>;
-      TRY(set_smem(ik, ism));
-      ik<<<NB / kTiB, 256, ism, c->stream>>>(reinterpret_cast<const float2*>(W), ld, k0, ncols, c->linv.as<float>(),
-                                     (long)NB * NB);
-      LAUNCH_CHECK();
-      auto gk = swap_gather_kernel<NB, CW, NT>;
-      const size_t gsm = (size_t)CW * (NB + 1) * sizeof(float2) + (size_t)CW * NB * sizeof(float2);
-      TRY(set_smem(gk, gsm));
-      gk<<<cdiv_u(N - k0 - ncols, CW), NT, gsm, c->stream>>>(reinterpret_cast<float2*>(W), ld, k0, ncols,
-                                                              sw.top_src, sw.extra_dst, sw.extra_src,
-                                                              sw.n_extra, k0 + ncols, N, bop, plane);
-      LAUNCH_CHECK();
-      if (tc_update(c->tcplan, c->op_linv, 0, 0, c->op_bop, 0, 0, NB,
-                    reinterpret_cast<float2*>(W) + k0 + (size_t)(k0 + ncols) * ld, ld, ncols, N - k0 - ncols, 128,
-                    c->stream))
-        return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
-      ++c->launches;
-      auto uk = u12_split_kernel<NB, CW, NT>;
-      uk<<<cdiv_u(N - k0 - ncols, CW), NT, 0, c->stream>>>(reinterpret_cast<const float2*>(W), ld, k0, ncols,
-                                                             k0 + ncols, N, bop, plane, c->lup.as<float>(),
-                                                             c->lup_ld, c->lup_plane, growth);
-      LAUNCH_CHECK();
-    } else if (!mixed) {
-      TRY(trsm(k0, ncols, sw, k0 + ncols, N, 0));
-    } else {
-      constexpr int CW = 32;
-      auto tk = trsm_lower_kernel<T, NB, CW, NT>;
-      size_t tsm = (size_t)CW * (NB + 1) * sizeof(T) + (size_t)CW * NB * sizeof(T);
-      TRY(set_smem(tk, tsm));
-      TrsmArgs<T> ta{};
-      ta.W = W;
-      ta.ld = ld;
-      ta.k0 = k0;
-      ta.ncols = ncols;
-      ta.top_src = sw.top_src;
-      ta.extra_dst = sw.extra_dst;
-      ta.extra_src = sw.extra_src;
-      ta.n_extra = sw.n_extra;
-      ta.X = W;
-      ta.ldx = ld;
-      ta.c_begin = k0 + ncols;
-      ta.c_end = N;
-      ta.growth_bits = growth;
-      // U12 also as the B operand of the trailing update and into the LU planes
-      ta.bop = bop;
-      ta.bop_plane = plane;
-      ta.bop_col0 = k0 + ncols;
-      ta.lup = c->lup.as<float>();
-      ta.lup_ld = c->lup_ld;
-      ta.lup_plane = c->lup_plane;
-      tk<<<cdiv_u(N - k0 - ncols, CW), NT, tsm, c->stream>>>(ta);
-      LAUNCH_CHECK();
-    }
+    TRY(trsm(k0, ncols, sw, k0 + ncols, N, 0));
     // trailing update A22 -= L21 U12
     const int M2 = N - k0 - ncols;
     if (mixed) {
@@ -2450,7 +2399,7 @@ int hprmat_b200_destroy(hprmat_b200_ctx* c) {
   cudaStreamSynchronize(c->stream);
   DevBuf* bufs[] = {&c->mesh, &c->W, &c->A64, &c->X, &c->X64, &c->R64, &c->B64, &c->V, &c->Z, &c->gm,
                     &c->swaps, &c->ipiv, &c->stage, &c->status, &c->ops, &c->inv, &c->chan, &c->rmat,
-                    &c->zwork, &c->cpot, &c->cu, &c->lup, &c->rop, &c->rsurf, &c->vt, &c->rlo, &c->linv,
+                    &c->zwork, &c->cpot, &c->cu, &c->lup, &c->rop, &c->rsurf, &c->vt, &c->rlo,
                     &c->wfx, &c->wfz, &c->wfc, &c->wfcf, &c->fpbuf};
   for (DevBuf* b : bufs) b->release();
   for (hprmat_b200_ctx* w : c->scan_workers) hprmat_b200_destroy(w);
@@ -4251,8 +4200,8 @@ int hprmat_b200_dev_set_tuning(hprmat_b200_ctx* c, const char* key, int value) {
     c->wave_enabled = value != 0;
     return HPRMAT_B200_OK;
   }
-  if (strcmp(key, "tc_trsm") == 0) {
-    c->tc_trsm = value != 0;
+  if (strcmp(key, "tc_trsm") == 0) {  // U12 has one implementation now; both values stay accepted
+    (void)value;
     return HPRMAT_B200_OK;
   }
   if (strcmp(key, "wave_sb") == 0) {

@@ -56,7 +56,7 @@ int hprmat_b200_dev_counters(hprmat_b200_ctx* ctx, unsigned long long* launches,
                       (0: 4, and explicit inverses of the whole factors up to 10 blocks); takes
                       effect at the next factorisation;
      "wave"           wavefront solves on/off (1);
-     "tc_trsm"        U12 by a tensor-core product with L11^-1 (1) or by substitution (0);
+     "tc_trsm"        accepted without effect: U12 is formed by substitution in registers;
      "panel_rpc_min"  fewest panel rows per CTA (32);
      "panel_cluster"  panels that fit in one cluster of at most 16 CTAs exchange pivots in
                       distributed shared memory (1) or always through global memory (0);
