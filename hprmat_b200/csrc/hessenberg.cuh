@@ -255,107 +255,75 @@ constexpr int kHbB = 32;           // panel width
 
 
 // The column step runs on one thread-block cluster (G = 8 or 16 CTAs of kHbCT threads, CTA q
-// holding rows [q rpc, (q + 1) rpc) of x in shared memory); its three sums over all rows are one
+// holding rows [q rpc, (q + 1) rpc) of x in shared memory); its two sums over all rows are one
 // partial per CTA in shared memory, summed by every CTA through the cluster's distributed shared
 // memory after a hardware cluster barrier.  The GEMV that follows each column needs the
-// bandwidth of all SMs and is a launch of its own (hb_gemv_kernel).
-constexpr int kHbCT = 256;
-// The loops over the panel's earlier columns j < n (n runtime, at most kHbB) load in groups of 8
-// predicated loads (zero beyond n) issued together, so that their L2 latencies overlap.
-constexpr int kHbGrp = 8;
+// bandwidth of all SMs and is a launch of its own (hb_gemv_kernel); the products V^H u, which
+// nothing needs before the next column step, are extra CTAs of that launch instead of a third sum.
+// Both kernels are launched with programmatic serialisation: each is resident before the one
+// before it has ended and waits for its end (griddepcontrol.wait) before it reads anything.
+// A step is a chain of L2 latencies and barriers: four lanes share a row and split the earlier
+// columns, so that all loads of a row are in flight at once.  Measured, one column with its GEMV over the
+// reductions of N = 720, 1980 and 3840: 32 -> 25 us.
+constexpr int kHbCT = 512;
+constexpr int kHbParts = 4;  // lanes of a row
+constexpr int kHbPer = kHbB / kHbParts;
 
-// acc -= sum_{j < n} Y[j * ldy] * s[j]  (column stride ldy; s in shared memory)
-__device__ __forceinline__ void hb_sub_cols(double2& acc, const double2* Y, long ldy, const double2* s, int n) {
+// sum over the lanes of a row (lane bits 3 and 4)
+__device__ __forceinline__ double2 hb_row_sum(double2 v) {
 #pragma unroll
-  for (int j0 = 0; j0 < kHbB; j0 += kHbGrp) {
-    if (j0 >= n) break;
-    double2 y[kHbGrp];
-#pragma unroll
-    for (int q = 0; q < kHbGrp; ++q) y[q] = j0 + q < n ? Y[(size_t)(j0 + q) * ldy] : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int q = 0; q < kHbGrp; ++q)
-      if (j0 + q < n) cfms(acc, y[q], s[j0 + q]);
+  for (int o = 8; o <= 16; o <<= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
   }
+  return v;
 }
-
-
-// acc1 -= sum_{j < n} Y[j * ldy] s1[j] and acc2 -= sum_{j < n} Y[j * ldy] s2[j], one load of each Y
-__device__ __forceinline__ void hb_sub_cols2(double2& acc1, const double2* s1, double2& acc2, const double2* s2,
-                                             const double2* Y, long ldy, int n) {
+// sum over 16 consecutive lanes
+__device__ __forceinline__ double2 hb_sum16(double2 v) {
 #pragma unroll
-  for (int j0 = 0; j0 < kHbB; j0 += kHbGrp) {
-    if (j0 >= n) break;
-    double2 y[kHbGrp];
-#pragma unroll
-    for (int q = 0; q < kHbGrp; ++q) y[q] = j0 + q < n ? Y[(size_t)(j0 + q) * ldy] : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int q = 0; q < kHbGrp; ++q)
-      if (j0 + q < n) {
-        cfms(acc1, y[q], s1[j0 + q]);
-        cfms(acc2, y[q], s2[j0 + q]);
-      }
+  for (int o = 8; o > 0; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
   }
+  return v;
+}
+__device__ __forceinline__ void hb_pdl_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 namespace cgh = cooperative_groups;
 
 // out[j] = sum over rows r in [rlo, rhi) of conj(V[(k + j), r]) vec[r - r0], j < n (Vk = V + k ldv;
-// vec and out in shared memory): warp w takes j = 4w .. 4w + 3 over all the rows (lanes on
+// vec and out in shared memory): warp w takes J columns j = J w .. over all the rows (lanes on
 // consecutive rows), then sums across its lanes.
-static_assert((kHbCT / 32) * 4 >= kHbB, "four columns per warp cover the panel");
-__device__ void hb_cta_dots(const double2* Vk, long ldv, const double2* vec, int rlo, int rhi, int r0, int n,
-                            double2* out) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jb = warp * 4;
-  if (jb < n) {
-    double2 acc[4];
+template <int J>
+__device__ __forceinline__ void hb_dots(const double2* Vk, long ldv, const double2* vec, int rlo, int rhi, int r0, int n,
+                                        double2* out, int ostride) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jb = warp * J;
+  if (jb >= n) return;
+  double2 acc[J];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc[e] = make_double2(0.0, 0.0);
+  for (int e = 0; e < J; ++e) acc[e] = make_double2(0.0, 0.0);
 #pragma unroll 4
-    for (int r = rlo + lane; r < rhi; r += 32) {
-      const double2 xr = vec[r - r0];
+  for (int r = rlo + lane; r < rhi; r += 32) {
+    const double2 xr = vec[r - r0];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const double2 v = jb + e < n ? Vk[(size_t)(jb + e) * ldv + r] : make_double2(0.0, 0.0);
-        cfma(acc[e], make_double2(v.x, -v.y), xr);
-      }
+    for (int e = 0; e < J; ++e) {
+      const double2 v = jb + e < n ? Vk[(size_t)(jb + e) * ldv + r] : make_double2(0.0, 0.0);
+      cfma(acc[e], make_double2(v.x, -v.y), xr);
     }
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      for (int o = 16; o > 0; o >>= 1) {
-        acc[e].x += __shfl_xor_sync(0xffffffffu, acc[e].x, o);
-        acc[e].y += __shfl_xor_sync(0xffffffffu, acc[e].y, o);
-      }
-    if (lane == 0)
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (jb + e < n) out[jb + e] = acc[e];
   }
-  __syncthreads();
-}
-
-// tot[j] = sum over the cluster's ranks g < G of rank g's mine[j], j < n (tot shared; red: shared
-// [kHbCT / 32][32]).  Thread t reads ranks t / 32, t / 32 + 8, .. of j = t % 32: the remote loads of
-// all ranks are in flight together.
-__device__ void hb_cluster_sum(const cgh::cluster_group& cl, int G, double2* mine, int n, double2* red, double2* tot) {
-  const int j = threadIdx.x & 31, g0 = threadIdx.x >> 5;
-  double2 t = make_double2(0.0, 0.0);
-  if (j < n)
-    for (int g = g0; g < G; g += kHbCT / 32) {
-      const double2 m = cl.map_shared_rank(mine, (unsigned)g)[j];
-      t.x += m.x;
-      t.y += m.y;
+#pragma unroll
+  for (int e = 0; e < J; ++e)
+    for (int o = 16; o > 0; o >>= 1) {
+      acc[e].x += __shfl_xor_sync(0xffffffffu, acc[e].x, o);
+      acc[e].y += __shfl_xor_sync(0xffffffffu, acc[e].y, o);
     }
-  red[g0 * 32 + j] = t;
-  __syncthreads();
-  if ((int)threadIdx.x < n) {
-    double2 s = red[threadIdx.x];
-    for (int w = 1; w < kHbCT / 32; ++w) {
-      s.x += red[w * 32 + threadIdx.x].x;
-      s.y += red[w * 32 + threadIdx.x].y;
-    }
-    tot[threadIdx.x] = s;
-  }
-  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int e = 0; e < J; ++e)
+      if (jb + e < n) out[(size_t)(jb + e) * ostride] = acc[e];
 }
 
 struct HbColArgs {
@@ -371,111 +339,168 @@ struct HbColArgs {
   double2* V;            // reflector store (ldv)
   long ldv;
   double2* T;            // kHbB x kHbB of this panel
-  double2* s;            // kHbB: V[:, <i]^H u_i of the last column done (rank 0 writes it)
+  double2* flag;         // 2 where the last column's reflector is not the identity, else 0 (rank 0)
+  const double2* spart;  // V[:, <iy]^H u by GEMV chunk: spart[j * sld + ch]
+  int sld;
 };
 
-// (a) iy >= 0: Y[r, iy] = 2 (p_r - Y[r, <iy] s), p_r the GEMV chunk sums, s of column iy.
+// (a) iy >= 0: s = V[:, <iy]^H u and T[:, iy] (rank 0 stores it); Y[r, iy] = 2 (p_r - Y[r, <iy] s),
+// p_r the GEMV chunk sums.
 // (b) ix >= 0, column c = k + ix: x_r = A[r, c] - Y[r, <ix] conj(V[c, k + <ix]); w = V[k+1.., <ix]^H x;
-// z = T^H w; x[k+1..] -= V z; the reflector of x[c+1..] into V[:, c] and A[:, c]; s = V[:, <ix]^H u
-// and T[:, ix] (rank 0).  With both, ix = iy + 1, and one pass over Y[r, <iy] serves (a) and (b).
+// z = T^H w; x[k+1..] -= V z; the reflector of x[c+1..] into V[:, c] and A[:, c].
+// With both, ix = iy + 1, and one pass over Y[r, <iy] serves (a) and (b).
 // Dynamic shared memory: rpc complex (x).
+static_assert(kHbCT == 16 * kHbB && kHbB == 32, "16 lanes per panel column");
 __global__ void __launch_bounds__(kHbCT) hb_col_cluster_kernel(HbColArgs a) {
   extern __shared__ __align__(16) double2 xs[];
   __shared__ double2 mine[kHbB];  // this CTA's partial sums, read by the whole cluster
   __shared__ double2 tot[kHbB], zv[kHbB], cv[kHbB], sv[kHbB];
   __shared__ double2 Ts[kHbB * kHbB];  // T of the panel (columns < ix are final)
-  __shared__ double2 red[kHbCT];
   __shared__ double mine_ss, rd[kHbCT / 32], sst_s;
   __shared__ double2 mine_x0, x0_s;
   cgh::cluster_group cl = cgh::this_cluster();
   const int G = (int)cl.num_blocks(), q = (int)cl.block_rank();
   const int tid = threadIdx.x, N = a.N, k = a.k;
+  const int lane = tid & 31, part = lane >> 3;
   const int r0 = q * a.rpc, r1 = min(N, r0 + a.rpc);
+  const int rfirst = r0 + (tid >> 5) * 8 + (lane & 7);  // this thread's rows: every 8 * warps-th
+  constexpr int kRowStep = kHbCT / kHbParts;
   const int i = a.ix, c = k + i;
-  if (tid < a.iy) sv[tid] = a.s[tid];
+  const int j16 = tid >> 4, l16 = tid & 15;  // 16 lanes per panel column
+  hb_pdl_start();
+  {
+    double2 t = make_double2(0.0, 0.0);
+    if (j16 < a.iy)
+      for (int ch = l16; ch < a.nchunk; ch += 16) {
+        const double2 v = a.spart[(size_t)j16 * a.sld + ch];
+        t.x += v.x;
+        t.y += v.y;
+      }
+    t = hb_sum16(t);
+    if (l16 == 0) sv[j16] = t;
+  }
   if (tid < i) {
     const double2 vc = a.V[(size_t)(k + tid) * a.ldv + c];
     cv[tid] = make_double2(vc.x, -vc.y);
   }
-  if (i > 0)
-    for (int e = tid; e < kHbB * i; e += kHbCT) Ts[e] = a.T[e];
+  for (int e = tid; e < kHbB * a.iy; e += kHbCT) Ts[e] = a.T[e];
   __syncthreads();
-  for (int r = r0 + tid; r < r1; r += kHbCT) {
-    double2 xr = i >= 0 ? a.A[(size_t)c * a.lda + r] : make_double2(0.0, 0.0);
+  if (a.iy >= 0) {
+    // T[:, iy]: rows < iy from -2 T[<iy, <iy] s, row iy = 2 (or 0 for an identity reflector), rest 0
+    double2 t = make_double2(0.0, 0.0);
+    for (int m = j16 + l16; m < a.iy; m += 16) cfma(t, Ts[m * kHbB + j16], sv[m]);
+    t = hb_sum16(t);
+    if (l16 == 0) {
+      t = j16 < a.iy ? make_double2(-2.0 * t.x, -2.0 * t.y) : (j16 == a.iy ? a.flag[0] : make_double2(0.0, 0.0));
+      Ts[a.iy * kHbB + j16] = t;
+      if (q == 0) a.T[(size_t)a.iy * kHbB + j16] = t;
+    }
+  }
+  for (int rb = rfirst; rb - (lane & 7) < r1; rb += kRowStep) {  // the bound is the same for a warp
+    const bool in = rb < r1;
+    const int r = in ? rb : r1 - 1;
+    const double2 ar = i >= 0 ? a.A[(size_t)c * a.lda + r] : make_double2(0.0, 0.0);
+    double2 xr = make_double2(0.0, 0.0);
     if (a.iy >= 0) {
-      double pr[4] = {0.0, 0.0, 0.0, 0.0}, pi[4] = {0.0, 0.0, 0.0, 0.0};
-      int ch = 0;
-      for (; ch + 3 < a.nchunk; ch += 4) {
-        double2 t[4];
+      double2 y[kHbPer];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) t[e] = a.part[(size_t)(ch + e) * N + r];
+      for (int e = 0; e < kHbPer; ++e) {
+        const int j = part + kHbParts * e;
+        y[e] = j < a.iy ? a.Y[(size_t)j * a.ldy + r] : make_double2(0.0, 0.0);
+      }
+      double2 p = make_double2(0.0, 0.0);
+#pragma unroll 4
+      for (int ch = part; ch < a.nchunk; ch += kHbParts) {
+        const double2 t = a.part[(size_t)ch * N + r];
+        p.x += t.x;
+        p.y += t.y;
+      }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          pr[e] += t[e].x;
-          pi[e] += t[e].y;
+      for (int e = 0; e < kHbPer; ++e) {
+        const int j = part + kHbParts * e;
+        if (j < a.iy) {
+          cfms(p, y[e], sv[j]);
+          if (i >= 0) cfms(xr, y[e], cv[j]);
         }
       }
-      for (; ch < a.nchunk; ++ch) {
-        const double2 t = a.part[(size_t)ch * N + r];
-        pr[0] += t.x;
-        pi[0] += t.y;
-      }
-      double2 p = make_double2(pr[0] + pr[1] + pr[2] + pr[3], pi[0] + pi[1] + pi[2] + pi[3]);
-      if (i >= 0)
-        hb_sub_cols2(p, sv, xr, cv, a.Y + r, a.ldy, a.iy);
-      else
-        hb_sub_cols(p, a.Y + r, a.ldy, sv, a.iy);
-      const double2 y = make_double2(2.0 * p.x, 2.0 * p.y);
-      a.Y[(size_t)a.iy * a.ldy + r] = y;
-      if (i >= 0) cfms(xr, y, cv[a.iy]);
+      p = hb_row_sum(p);
+      xr = hb_row_sum(xr);
+      const double2 yn = make_double2(2.0 * p.x, 2.0 * p.y);
+      if (in && part == 0) a.Y[(size_t)a.iy * a.ldy + r] = yn;
+      if (i >= 0) cfms(xr, yn, cv[a.iy]);
     }
-    if (i >= 0) xs[r - r0] = xr;
+    if (in && i >= 0 && part == 0) xs[r - r0] = make_double2(ar.x + xr.x, ar.y + xr.y);
   }
   if (i < 0) return;  // uniform: no CTA of the cluster reads another's shared memory
   __syncthreads();
   if (i > 0) {
-    hb_cta_dots(a.V + (size_t)k * a.ldv, a.ldv, xs, max(r0, k + 1), r1, r0, i, mine);
+    hb_dots<2>(a.V + (size_t)k * a.ldv, a.ldv, xs, max(r0, k + 1), r1, r0, i, mine, 1);
     cl.sync();
-    hb_cluster_sum(cl, G, mine, i, red, tot);
-    // z_j = sum_{l <= j} conj(T[l, j]) w_l
-    if (tid < i) {
+    {  // the cluster's sums: 16 lanes per column, one rank each
+      double2 t = make_double2(0.0, 0.0);
+      if (j16 < i && l16 < G) t = cl.map_shared_rank(mine, (unsigned)l16)[j16];
+      t = hb_sum16(t);
+      if (l16 == 0) tot[j16] = t;
+    }
+    __syncthreads();
+    {  // z_j = sum_{l <= j} conj(T[l, j]) w_l
       double2 acc = make_double2(0.0, 0.0);
-      for (int l = 0; l <= tid; ++l) {
-        const double2 t = Ts[tid * kHbB + l];
-        cfma(acc, make_double2(t.x, -t.y), tot[l]);
-      }
-      zv[tid] = acc;
+      if (j16 < i)
+        for (int l = l16; l <= j16; l += 16) {
+          const double2 t = Ts[j16 * kHbB + l];
+          cfma(acc, make_double2(t.x, -t.y), tot[l]);
+        }
+      acc = hb_sum16(acc);
+      if (l16 == 0) zv[j16] = acc;
     }
     __syncthreads();
   }
   double ss = 0.0;
-  for (int r = r0 + tid; r < r1; r += kHbCT) {
+  for (int rb = rfirst; rb - (lane & 7) < r1; rb += kRowStep) {
+    const bool in = rb < r1;
+    const int r = in ? rb : r1 - 1;
     double2 v = xs[r - r0];
-    if (i > 0 && r >= k + 1) {
-      hb_sub_cols(v, a.V + (size_t)k * a.ldv + r, a.ldv, zv, i);
-      xs[r - r0] = v;
+    if (i > 0) {
+      double2 y[kHbPer], d = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int e = 0; e < kHbPer; ++e) {
+        const int j = part + kHbParts * e;
+        y[e] = j < i ? a.V[(size_t)(k + j) * a.ldv + r] : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int e = 0; e < kHbPer; ++e) {
+        const int j = part + kHbParts * e;
+        if (j < i) cfms(d, y[e], zv[j]);
+      }
+      d = hb_row_sum(d);
+      if (r >= k + 1) {
+        v.x += d.x;
+        v.y += d.y;
+        if (in && part == 0) xs[r - r0] = v;  // after the row's lanes have read it (hb_row_sum)
+      }
     }
-    if (r > c) ss += v.x * v.x + v.y * v.y;
-    if (r == c + 1) mine_x0 = v;
+    if (in && part == 0) {
+      if (r > c) ss += v.x * v.x + v.y * v.y;
+      if (r == c + 1) mine_x0 = v;
+    }
   }
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if ((tid & 31) == 0) rd[tid >> 5] = ss;
+  if (lane == 0) rd[tid >> 5] = ss;
   __syncthreads();
-  if (tid == 0) {
-    double t = 0.0;
-    for (int w = 0; w < kHbCT / 32; ++w) t += rd[w];
-    mine_ss = t;
+  if (tid < 32) {
+    double t = tid < kHbCT / 32 ? rd[tid] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (tid == 0) mine_ss = t;
   }
-  cl.sync();  // also: every CTA has read the w partials
+  cl.sync();
   if (tid < 32) {
     double v = tid < G ? *cl.map_shared_rank(&mine_ss, (unsigned)tid) : 0.0;
+    if (tid == 31) x0_s = *cl.map_shared_rank(&mine_x0, (unsigned)((c + 1) / a.rpc));
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (tid == 0) {
-      sst_s = v;
-      x0_s = *cl.map_shared_rank(&mine_x0, (unsigned)((c + 1) / a.rpc));
-    }
+    if (tid == 0) sst_s = v;
   }
   __syncthreads();
+  cl.barrier_arrive();  // this CTA's last remote reads are done
   const double sst = sst_s;
   const double2 x0 = x0_s;
   const double a0 = hypot(x0.x, x0.y);
@@ -501,44 +526,32 @@ __global__ void __launch_bounds__(kHbCT) hb_col_cluster_kernel(HbColArgs a) {
     }
     a.V[(size_t)c * a.ldv + r] = u;
     a.A[(size_t)c * a.lda + r] = r <= c ? xr : (r == c + 1 ? gamma : make_double2(0.0, 0.0));
-    xs[r - r0] = u;  // x is done with; u for the sums below
   }
-  __syncthreads();
-  // the w partials in mine were read by every CTA before the barrier after the norm
-  if (i > 0) hb_cta_dots(a.V + (size_t)k * a.ldv, a.ldv, xs, max(r0, c + 1), r1, r0, i, mine);
-  cl.sync();
-  if (q == 0) {
-    hb_cluster_sum(cl, G, mine, i, red, tot);
-    if (tid < i) a.s[tid] = tot[tid];
-    // T[:, i]: rows < i from -2 T[<i, <i] s, row i = 2 (or 0 for an identity reflector), rest 0
-    if (tid < kHbB) {
-      double2 t = make_double2(0.0, 0.0);
-      if (tid < i) {
-        for (int m = tid; m < i; ++m) cfma(t, Ts[m * kHbB + tid], tot[m]);
-        t = make_double2(-2.0 * t.x, -2.0 * t.y);
-      } else if (tid == i) {
-        t = make_double2(sst > 0.0 ? 2.0 : 0.0, 0.0);
-      }
-      a.T[(size_t)i * kHbB + tid] = t;
-    }
-  }
-  cl.sync();  // no CTA leaves while rank 0 reads its partials
+  if (q == 0 && tid == 0) a.flag[0] = make_double2(sst > 0.0 ? 2.0 : 0.0, 0.0);
+  cl.barrier_wait();  // no CTA leaves while another reads its partials
 }
 
 // The GEMV of column c: part[ch * N + r] = sum over the 256 columns j of chunk ch (from c + 1) of
 // A[r, j] u_j, u = V[:, c].  A CTA takes 32 rows and one chunk; warp w its 32 columns w * 32 ..,
-// 16 loads in flight per thread; the 8 warps' sums are added in shared memory.
+// 16 loads in flight per thread; the 8 warps' sums are added in shared memory.  The last column of
+// CTAs forms the chunk's part of V[:, k + <i]^H u: spart[j * sld + ch] (Vk = V + k ldv).
 constexpr int kHbGemvCols = 256;
-__global__ void __launch_bounds__(256) hb_gemv_kernel(const double2* __restrict__ A, long lda, int N, int c,
-                                                      const double2* __restrict__ u, double2* part) {
+__global__ void __launch_bounds__(256) hb_gemv_kernel(const double2* A, long lda, int N, int c,
+                                                      const double2* u, double2* part, const double2* Vk, long ldv,
+                                                      int i, double2* spart, int sld) {
   __shared__ double2 us[kHbGemvCols];
   __shared__ double2 red[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 32 + lane;
   const int j0 = c + 1 + blockIdx.y * kHbGemvCols;
   const int j1 = min(j0 + kHbGemvCols, N);
+  hb_pdl_start();
   us[threadIdx.x] = j0 + (int)threadIdx.x < j1 ? u[j0 + threadIdx.x] : make_double2(0.0, 0.0);
   __syncthreads();
+  if (blockIdx.x + 1 == gridDim.x) {
+    hb_dots<4>(Vk, ldv, us, j0, j1, j0, i, spart + blockIdx.y, sld);
+    return;
+  }
   double pr[4] = {0.0, 0.0, 0.0, 0.0}, pi[4] = {0.0, 0.0, 0.0, 0.0};
   const int jw = j0 + warp * 32;
   if (row < N && jw + 32 <= j1) {
@@ -548,7 +561,7 @@ __global__ void __launch_bounds__(256) hb_gemv_kernel(const double2* __restrict_
     for (int b = 0; b < 32; b += 16) {
       double2 av[16];
 #pragma unroll
-      for (int e = 0; e < 16; ++e) av[e] = __ldg(Ar + (size_t)(b + e) * lda);
+      for (int e = 0; e < 16; ++e) av[e] = Ar[(size_t)(b + e) * lda];
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
         const double2 uu = us[warp * 32 + b + e];
@@ -601,34 +614,36 @@ __global__ void splitk_sum_kernel(double2* C, long ldc, int M, int Nc, const dou
 }
 
 // Per panel (b columns at k): VH = V[:, k..k+b)^H (b x N, column-major, ld kHbB) and
-// VT = -V T^H (conj_t) or -V T (N x kHbB, column-major, ld N) for rows r of the grid.
-__global__ void hb_prep_kernel(int N, int k, int b, const double2* __restrict__ V, long ldv,
-                               const double2* __restrict__ T, double2* VH, double2* VT, bool conj_t) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= N) return;
-  double2 v[kHbB];
-#pragma unroll
-  for (int j = 0; j < kHbB; ++j) v[j] = j < b ? V[(size_t)(k + j) * ldv + r] : make_double2(0.0, 0.0);
-#pragma unroll
-  for (int j = 0; j < kHbB; ++j) VH[(size_t)r * kHbB + j] = make_double2(v[j].x, -v[j].y);
-  // (V T^H)[r, j] = sum_{l >= j} V[r, l] conj(T[j, l]);  (V T)[r, j] = sum_{l <= j} V[r, l] T[l, j].
-  // Both loops fully unrolled (v stays in registers); V is zero in the columns l >= b.
-#pragma unroll
-  for (int j = 0; j < kHbB; ++j) {
-    double2 acc = make_double2(0.0, 0.0);
-    if (conj_t) {
-#pragma unroll
-      for (int l = j; l < kHbB; ++l) {
-        const double2 t = l < b ? T[(size_t)l * kHbB + j] : make_double2(0.0, 0.0);
-        cfma(acc, v[l], make_double2(t.x, -t.y));
-      }
-    } else {
-#pragma unroll
-      for (int l = 0; l <= j; ++l) cfma(acc, v[l], T[(size_t)j * kHbB + l]);
-    }
-    if (j >= b) acc = make_double2(0.0, 0.0);
-    VT[(size_t)j * N + r] = make_double2(-acc.x, -acc.y);
+// VT = -V T^H (conj_t) or -V T (N x kHbB, column-major, ld N).  A CTA takes kHbPrepRows rows, a thread
+// one element of VT, with T and the rows of V in shared memory (one thread per row, T from L2:
+// a chain of loads on 30 CTAs at N = 3840: 34 us, against less than 5).
+constexpr int kHbPrepRows = 16;
+__global__ void __launch_bounds__(kHbPrepRows * kHbB) hb_prep_kernel(int N, int k, int b, const double2* __restrict__ V,
+                                                                     long ldv, const double2* __restrict__ T,
+                                                                     double2* VH, double2* VT, bool conj_t) {
+  __shared__ double2 Ts[kHbB * kHbB], vs[kHbB][kHbPrepRows + 1];
+  constexpr int NT = kHbPrepRows * kHbB;
+  const int tid = threadIdx.x, rb = blockIdx.x * kHbPrepRows;
+  const int rr = tid % kHbPrepRows, j = tid / kHbPrepRows, r = rb + rr;
+  vs[j][rr] = j < b && r < N ? V[(size_t)(k + j) * ldv + r] : make_double2(0.0, 0.0);
+  for (int e = tid; e < kHbB * kHbB; e += NT) Ts[e] = e < b * kHbB ? T[e] : make_double2(0.0, 0.0);
+  __syncthreads();
+  {
+    const int jj = tid % kHbB, r2 = tid / kHbB;
+    const double2 v = vs[jj][r2];
+    if (rb + r2 < N) VH[(size_t)(rb + r2) * kHbB + jj] = make_double2(v.x, -v.y);
   }
+  // (V T^H)[r, j] = sum_{l >= j} V[r, l] conj(T[j, l]);  (V T)[r, j] = sum_{l <= j} V[r, l] T[l, j]
+  double2 acc = make_double2(0.0, 0.0);
+  if (conj_t) {
+#pragma unroll 8
+    for (int l = j; l < b; ++l) cfma(acc, vs[l][rr], make_double2(Ts[l * kHbB + j].x, -Ts[l * kHbB + j].y));
+  } else {
+#pragma unroll 8
+    for (int l = 0; l <= j; ++l) cfma(acc, vs[l][rr], Ts[j * kHbB + l]);
+  }
+  if (j >= b) acc = make_double2(0.0, 0.0);
+  if (r < N) VT[(size_t)j * N + r] = make_double2(-acc.x, -acc.y);
 }
 
 // ---------------------------------------------------------------- per-energy Hessenberg solves

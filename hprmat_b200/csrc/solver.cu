@@ -2881,7 +2881,9 @@ static int hess_reduce_blocked(hprmat_b200_ctx* c, double2* A, long ld, int N, d
   double2* VH = c->hbVH.as<double2>();
   double2* VT = c->hbVT.as<double2>();
   double2* W = c->hbW.as<double2>();
-  TRY(c->hbS.ensure((size_t)kHbB * sizeof(double2)));
+  const int sld = cdiv_u(N, kHbGemvCols);
+  TRY(c->hbS.ensure((size_t)(kHbB * sld + 1) * sizeof(double2)));
+  double2* spart = c->hbS.as<double2>();
   double2* part = c->hPart.as<double2>();
   // the column step's cluster: 16 CTAs where the GPU holds such a cluster, else 8 (portable)
   if (c->hb_cluster == 0) {
@@ -2924,20 +2926,24 @@ static int hess_reduce_blocked(hprmat_b200_ctx* c, double2* A, long ld, int N, d
   ca.ldy = N;
   ca.V = V;
   ca.ldv = ld;
-  ca.s = c->hbS.as<double2>();
+  ca.spart = spart;
+  ca.sld = sld;
+  ca.flag = spart + (size_t)kHbB * sld;
   auto column_step = [&]() -> int {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(Gc);
     cfg.blockDim = dim3(kHbCT);
     cfg.dynamicSmemBytes = xsm;
     cfg.stream = c->stream;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = Gc;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, hb_col_cluster_kernel, ca);
     if (e != cudaSuccess)
       return fail(HPRMAT_B200_ERR_CUDA, "Hessenberg column step (%d CTAs of %d rows): %s", Gc, rpc,
@@ -2985,8 +2991,19 @@ static int hess_reduce_blocked(hprmat_b200_ctx* c, double2* A, long ld, int N, d
     for (int i = 0; i < b; ++i) {
       const int col = k + i;
       const int nchunk = cdiv_u(N - col - 1, kHbGemvCols);
-      hb_gemv_kernel<<<dim3(cdiv_u(N, 32), nchunk), 256, 0, c->stream>>>(A, ld, N, col, V + (size_t)col * ld, part);
-      LAUNCH_CHECK();
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(cdiv_u(N, 32) + 1, nchunk);
+      cfg.blockDim = dim3(256);
+      cfg.stream = c->stream;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      HPR_CUDA_TRY(cudaLaunchKernelEx(&cfg, hb_gemv_kernel, (const double2*)A, ld, N, col,
+                                      (const double2*)(V + (size_t)col * ld), part,
+                                      (const double2*)(V + (size_t)k * ld), ld, i, spart, sld));
+      ++c->launches;
       ca.iy = i;
       ca.ix = i + 1 < b ? i + 1 : -1;
       ca.nchunk = nchunk;
@@ -2994,7 +3011,7 @@ static int hess_reduce_blocked(hprmat_b200_ctx* c, double2* A, long ld, int N, d
     }
     if (k + b < N) {
       const int nt = N - k - b;
-      hb_prep_kernel<<<cdiv_u(N, 128), 128, 0, c->stream>>>(N, k, b, V, ld, Tp, VH, VT, true);
+      hb_prep_kernel<<<cdiv_u(N, kHbPrepRows), kHbPrepRows * kHbB, 0, c->stream>>>(N, k, b, V, ld, Tp, VH, VT, true);
       LAUNCH_CHECK();
       // A[:, k+b ..] -= Y V[k+b .., ]^H
       TRY(gemm(N, nt, b, Y, N, VH + (size_t)(k + b) * kHbB, kHbB, A + (size_t)(k + b) * ld, ld));
@@ -3012,7 +3029,7 @@ static int hess_reduce_blocked(hprmat_b200_ctx* c, double2* A, long ld, int N, d
     const int k = p * kHbB, b = std::min(kHbB, ncols - k);
     const double2* Tp = c->hbT.as<double2>() + (size_t)p * kHbB * kHbB;
     const int m = N - k - 1;
-    hb_prep_kernel<<<cdiv_u(N, 128), 128, 0, c->stream>>>(N, k, b, V, ld, Tp, VH, VT, false);
+    hb_prep_kernel<<<cdiv_u(N, kHbPrepRows), kHbPrepRows * kHbB, 0, c->stream>>>(N, k, b, V, ld, Tp, VH, VT, false);
     LAUNCH_CHECK();
     HPR_CUDA_TRY(cudaMemsetAsync(W, 0, (size_t)kHbB * m * sizeof(double2), c->stream));
     TRY(gemm_splitk(b, m, m, VH + (size_t)(k + 1) * kHbB, kHbB, P + (k + 1) + (size_t)(k + 1) * ld, ld, W, kHbB));
@@ -3412,32 +3429,43 @@ int hprmat_b200_rmatrix_scan_shifted(hprmat_b200_ctx* c, int nblocks, const hprm
     if (w->profile) w->hess_ms[5] += ms_since(tfb);
     return HPRMAT_B200_OK;
   };
-  const int nw = std::max(1, std::min(c->hess_workers, nblocks));
+  // Blocks by the least loaded worker, largest first (cost ~ N^3 for the reduction plus
+  // nenergies N^2 nch for the energies), on nw workers.
+  std::vector<std::vector<int>> mine;
+  auto assign = [&](int nw) -> double {
+    std::vector<int> order(nblocks);
+    std::vector<double> cost(nblocks), load((size_t)nw, 0.0);
+    for (int b = 0; b < nblocks; ++b) {
+      order[b] = b;
+      const double n = (double)blocks[b].nch * nr;
+      cost[b] = n * n * n + (double)blocks[b].nenergies * n * n * blocks[b].nch;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+    mine.assign((size_t)nw, {});
+    for (const int b : order) {
+      const int i = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+      mine[i].push_back(b);
+      load[i] += cost[b];
+    }
+    return *std::max_element(load.begin(), load.end());
+  };
+  // The fewest workers whose largest share is within 10 % of that of all of them: blocks in flight
+  // beyond that only slow the largest one down, which the scan waits for (blocks of N = 720, 1980 and
+  // 3840 with 64 energies: 429 ms on one worker, 383 on two, 447 on three;
+  // twelve of N = 600 .. 1920: 455, 336, 294).
+  const int nw_max = std::max(1, std::min(c->hess_workers, nblocks));
+  const double best = assign(nw_max);
+  int nw = 1;
+  while (nw < nw_max && assign(nw) > 1.1 * best) ++nw;
+  if (nw == nw_max) assign(nw);
   if (nw == 1) {
     for (int b = 0; b < nblocks; ++b) TRY(run_block(c, b, &first_error, &err_msg));
   } else {
     // Several blocks in flight, one worker context (stream, buffers, host thread) each, so that
-    // one block's latency-bound reduction overlaps the others' GEMMs and solves.  Blocks go to
-    // the least loaded worker, largest first (cost ~ N^3 for the reduction plus
-    // nenergies N^2 nch for the energies); each worker gets its share of the batch budget.
+    // one block's latency-bound reduction overlaps the others' GEMMs and solves; each worker gets
+    // its share of the batch budget.
     TRY(scan_workers_ready(c, nw, nr, rmax));
     c->hess_steps_last = 0;
-    std::vector<std::vector<int>> mine((size_t)nw);
-    {
-      std::vector<int> order(nblocks);
-      std::vector<double> cost(nblocks), load((size_t)nw, 0.0);
-      for (int b = 0; b < nblocks; ++b) {
-        order[b] = b;
-        const double n = (double)blocks[b].nch * nr;
-        cost[b] = n * n * n + (double)blocks[b].nenergies * n * n * blocks[b].nch;
-      }
-      std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-      for (const int b : order) {
-        const int i = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        mine[i].push_back(b);
-        load[i] += cost[b];
-      }
-    }
     std::vector<int> status((size_t)nw, HPRMAT_B200_OK), ferr((size_t)nw, HPRMAT_B200_OK);
     std::vector<std::string> fail_msg((size_t)nw), emsg((size_t)nw);
     std::vector<std::thread> th;
