@@ -12,8 +12,8 @@
 //                           eliminate their rows.  Writes ipiv and the step's row-interchange
 //                           list.
 //   2. trsm_reg_kernel   -- applies the step's row interchanges to the columns right of the
-//      (trsm_lower_kernel)  panel (or to right-hand sides) and solves with the unit lower
-//                           diagonal block: U12 = L11^-1 P A12.
+//                           panel and solves with the unit lower diagonal block:
+//                           U12 = L11^-1 P A12.
 //   3. trailing update   -- A22 -= L21 U12 (cgemm_update_kernel here; the mixed path uses
 //                           the tcgen05 kernel of tc_gemm.cu).
 // Row interchanges are applied only to columns at or right of the current panel; the
@@ -363,68 +363,14 @@ struct TrsmArgs {
   int mode;          // 0: interchanges and solve; 1: interchanges only; 2: solve only (rows k0..)
 };
 
-template <typename T, int NB, int CW, int NT>
-__global__ void __launch_bounds__(NT) trsm_lower_kernel(TrsmArgs<T> a) {
-  using R = typename RealOf<T>::R;
-  constexpr int NBP = NB + 1;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* A = reinterpret_cast<T*>(smem_raw);  // [CW][NBP]
-  T* E = A + CW * NBP;                    // [CW][NB]
-  const int tid = threadIdx.x;
-  const int cb = a.c_begin + blockIdx.x * CW;
-  const int ncw = min(CW, a.c_end - cb);
-  if (ncw <= 0) return;
-  const int ncols = a.ncols;
-  const bool swap = a.mode != 2, solve = a.mode != 1;
-  const int ne = swap ? *a.n_extra : 0;
-  for (int idx = tid; idx < ncw * ncols; idx += NT) {
-    int j = idx % ncols, cc = idx / ncols;
-    A[cc * NBP + j] = a.X[(size_t)(swap ? a.top_src[j] : a.k0 + j) + (size_t)(cb + cc) * a.ldx];
-  }
-  for (int idx = tid; idx < ncw * ne; idx += NT) {
-    int e = idx % ne, cc = idx / ne;
-    E[cc * NB + e] = a.X[(size_t)a.extra_src[e] + (size_t)(cb + cc) * a.ldx];
-  }
-  __syncthreads();
-  for (int idx = tid; idx < ncw * ne; idx += NT) {
-    int e = idx % ne, cc = idx / ne;
-    a.X[(size_t)a.extra_dst[e] + (size_t)(cb + cc) * a.ldx] = E[cc * NB + e];
-  }
-  for (int j = 0; j < (solve ? ncols - 1 : 0); ++j) {
-    __syncthreads();
-    const int nr = ncols - j - 1;
-    const T* Lcol = a.W + (size_t)(a.k0 + j) * a.ld + a.k0;
-    for (int idx = tid; idx < nr * ncw; idx += NT) {
-      int i = j + 1 + idx % nr, cc = idx / nr;
-      T l = Lcol[i];
-      T v = A[cc * NBP + i];
-      cfms(v, l, A[cc * NBP + j]);
-      A[cc * NBP + i] = v;
-    }
-  }
-  __syncthreads();
-  R gmax = R(0);
-  for (int idx = tid; idx < ncw * ncols; idx += NT) {
-    int j = idx % ncols, cc = idx / ncols;
-    T v = A[cc * NBP + j];
-    a.X[(size_t)(a.k0 + j) + (size_t)(cb + cc) * a.ldx] = v;
-    gmax = fmax(gmax, cabs1(v));
-  }
-  if (a.growth_bits && solve) {
-    for (int o = 16; o > 0; o >>= 1) gmax = fmax(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
-    if ((tid & 31) == 0) atomicMax(a.growth_bits, mag_hi((double)gmax));
-  }
-}
-
-// trsm_lower_kernel with the right-hand sides in registers: LN = NB / 16 lanes share a column, lane g
+// Interchanges and substitution with the right-hand sides in registers: LN = NB / 16 lanes share a column, lane g
 // holding rows LN a + g in x[a], a < 16.  A step broadcasts x_k within the lanes of a column and
 // updates the rows below; L11 is staged in shared memory once per CTA, and a group of 2 NB threads
-// walks over blocks of 32 columns (one barrier and one L2 read of L's column per step in
-// trsm_lower_kernel, no barrier here).  x moves one register down every LN steps and its end takes the
+// walks over blocks of 32 columns (no barrier between the steps).  x moves one register down every LN steps and its end takes the
 // finished row, so that the code of LN steps serves several blocks of them and the rows are back in
-// place after 16; the displaced rows travel through the same shared memory meanwhile.  The operations
-// of trsm_lower_kernel in its order.
-// Measured, average over the steps: FP64, N = 4000 with NB = 64 41 -> 12 us.  Mixed, NB = 128, against
+// place after 16; the displaced rows travel through the same shared memory meanwhile.
+// Measured, average over the steps: FP64, N = 4000 with NB = 64, against one barrier and one L2 read of L's column
+// per step: 41 -> 12 us.  Mixed, NB = 128, against
 // the inverse of L11, a row gather, a tensor-core product and a split of its result as four launches:
 // N = 400 40 -> 22 us, N = 3000 46 -> 23, N = 6400 48 -> 27, N = 25600 66 -> 71 (0.3 % of that
 // factorisation); and no inverse enters U any more.  Bound by the chain of NB broadcasts and updates,

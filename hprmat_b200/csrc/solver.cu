@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -210,6 +211,10 @@ struct hprmat_b200_ctx {
   int hb_cluster = 0;  // CTAs of the Hessenberg column step's cluster (0: not chosen yet)
   // batched energy scans: worker contexts (own stream and buffers) and the blocks' potentials
   std::vector<hprmat_b200_ctx*> scan_workers;
+  // the LU's look-ahead: the next panel's stream and its events (factor_impl)
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_ev[3] = {nullptr, nullptr, nullptr};
+  int lookahead = 2048;  // fewest rows of a trailing matrix that is updated beside the next panel (0: never)
   std::vector<std::unique_ptr<DevBuf>> scan_cpot;
   std::vector<ScanTune> scan_tune;  // autotuner table, applied per unit by rmatrix_scan
   int wtrace_units = 0;
@@ -686,12 +691,8 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     ta.lup = mixed ? c->lup.as<float>() : nullptr;
     ta.lup_ld = c->lup_ld;
     ta.lup_plane = c->lup_plane;
-    if constexpr (sizeof(T) == sizeof(double2) && NB == 128) {  // L11 does not fit in shared memory
-      constexpr int CW = 32;
-      auto tk = trsm_lower_kernel<T, NB, CW, NT>;
-      const size_t tsm = (size_t)CW * (NB + 1) * sizeof(T) + (size_t)CW * NB * sizeof(T);
-      TRY(set_smem(tk, tsm));
-      tk<<<cdiv_u(c_end - c_begin, CW), NT, tsm, c->stream>>>(ta);
+    if constexpr (sizeof(T) == sizeof(double2) && NB == 128) {  // nor do the solves' diagonal blocks fit
+      return fail(HPRMAT_B200_ERR_CUDA, "FP64 block size 128: L11 does not fit in shared memory");
     } else {
       auto tk = trsm_reg_kernel<T, NB>;
       const unsigned blocks = cdiv_u(c_end - c_begin, kTrsmCols), ctas = (NB == 128 ? 1u : 2u) * (unsigned)c->nsm;
@@ -702,7 +703,67 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     LAUNCH_CHECK();
     return HPRMAT_B200_OK;
   };
+  // the largest rows per CTA of a cluster panel (shared memory of the opt-in limit, less the
+  // static arrays)
+  int rpc_max_c = 0;
+  const size_t static_c = (sizeof(T) == sizeof(double2) ? 20 : 12) * 1024;
+  while (rpc_max_c < kRegPanelRows && panel_reg_smem<T, NB>(rpc_max_c + 1) + static_c <= (size_t)c->smem_optin)
+    ++rpc_max_c;
+  // Look-ahead of the mixed path: the panel of step s + 1 needs only its own columns of step s's
+  // trailing update.  They are updated first; the panel then runs on a stream of its own, on the 16
+  // SMs of its cluster, and the update of the other columns beside it on the rest.  The update
+  // starts when the panel's first cluster is resident (a launch completion event: persistent CTAs
+  // placed first would leave no GPC with 16 free SMs), and the next step waits for both.
+  // Measured (factorisation alone, without -> with): N = 3000 6.89 -> 6.74 ms, 6400 21.5 -> 19.1, 12800 69.6
+  // -> 56.9, 25600 330 -> 303.  The line at 2048 rows: 1000 to 3000 measure alike (the panel hides 15 to
+  // 45 us of update there and pays 12 for the launch of its columns).  The same factors bit for bit.
+  int ahead_k0 = -1;  // step whose other columns are still to be updated
+  // trailing update of the columns j0 .. j1 right of the panel at k0, on at most max_grid CTAs (0: all)
+  auto update_columns = [&](int k0, int ncols, int j0, int j1, int max_grid) -> int {
+    const int k1 = k0 + ncols, M2 = N - k1;
+    const bool prof = c->profile && c->ev_used + 2 <= (int)c->ev.size();
+    if (prof) HPR_CUDA_TRY(cudaEventRecord(c->ev[c->ev_used], c->stream));
+    const int cap = c->tcplan.max_grid;
+    if (max_grid > 0) c->tcplan.max_grid = cap > 0 ? std::min(cap, max_grid) : max_grid;
+    const int e = tc_update(c->tcplan, c->op_lu, k0, k1, c->op_bop, 0, j0, NB,
+                            reinterpret_cast<float2*>(W) + k1 + (size_t)(k1 + j0) * ld, ld, M2, j1 - j0, 128, c->stream);
+    c->tcplan.max_grid = cap;
+    if (e) return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
+    ++c->launches;
+    if (prof) {
+      HPR_CUDA_TRY(cudaEventRecord(c->ev[c->ev_used + 1], c->stream));
+      c->ev_flops.push_back(8.0 * (double)M2 * (double)(j1 - j0) * (double)NB);
+      c->ev_used += 2;
+    }
+    return HPRMAT_B200_OK;
+  };
+  // SMs left to the panel of m rows: 16 for one cluster kernel.  Tall panels are 16-SM kernels and, between
+  // them, rank-16 updates of the panel on whatever is free, and take the SMs at which the panel and the
+  // update end together by the measured times in us: the sub-panels 20 + 10 per 8192 rows each, their
+  // updates 0.91 m / SMs, the trailing update 6.5e-4 m^2 / SMs.  N = 6400: 20.4 ms with 16 SMs left, 19.3
+  // with 64, 19.05 by this rule; N = 12800: 63.4, 61.3, 56.9; N = 25600: 306, 363, 303.
+  auto ahead_sms = [&](int m) -> int {
+    if (m <= 16 * rpc_max_c) return 16;
+    const double rows = m, subs = 40.0 + 8.0 * (20.0 + 10.0 * std::ceil(rows / 8192.0));
+    const int most = std::max(16, std::min(80, c->nsm / 2));
+    int r = 16;
+    while (r < most && 6.5e-4 * rows * rows / (c->nsm - r) < subs + 0.91 * rows / r) r += 4;
+    return r;
+  };
+  // after the first kernel of the panel beside which the update runs (launched with side_ev[1])
+  auto ahead_update = [&]() -> int {
+    HPR_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->side_ev[1], 0));
+    return update_columns(ahead_k0, NB, NB, N - ahead_k0 - NB, c->nsm - ahead_sms(N - ahead_k0 - NB));
+  };
+  auto ahead_join = [&]() -> int {  // after the panel's last kernel
+    if (ahead_k0 < 0) return HPRMAT_B200_OK;
+    ahead_k0 = -1;
+    HPR_CUDA_TRY(cudaEventRecord(c->side_ev[2], c->side));
+    HPR_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->side_ev[2], 0));
+    return HPRMAT_B200_OK;
+  };
   // after the panel of step s: row interchanges, U12 = L11^-1 P A12 and the trailing update
+  std::function<bool(int)> ahead_fits = [](int) { return false; };
   auto after_panel = [&](int s, int k0, int ncols, const StepSwaps& sw) -> int {
     (void)s;
     // row interchanges + U12 = L11^-1 A12
@@ -710,17 +771,13 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     // trailing update A22 -= L21 U12
     const int M2 = N - k0 - ncols;
     if (mixed) {
-      const bool prof = c->profile && c->ev_used + 2 <= (int)c->ev.size();
-      if (prof) HPR_CUDA_TRY(cudaEventRecord(c->ev[c->ev_used], c->stream));
-      if (tc_update(c->tcplan, c->op_lu, k0, k0 + ncols, c->op_bop, 0, 0, NB,
-                    reinterpret_cast<float2*>(W) + (k0 + ncols) + (size_t)(k0 + ncols) * ld, ld, M2, M2, 128,
-                    c->stream))
-        return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
-      ++c->launches;
-      if (prof) {
-        HPR_CUDA_TRY(cudaEventRecord(c->ev[c->ev_used + 1], c->stream));
-        c->ev_flops.push_back(8.0 * (double)M2 * (double)M2 * (double)NB);
-        c->ev_used += 2;
+      if (ahead_fits(k0 + ncols)) {  // now the next panel's columns only, the others beside that panel
+        TRY(update_columns(k0, ncols, 0, NB, 0));
+        HPR_CUDA_TRY(cudaEventRecord(c->side_ev[0], c->stream));
+        HPR_CUDA_TRY(cudaStreamWaitEvent(c->side, c->side_ev[0], 0));
+        ahead_k0 = k0;
+      } else {
+        TRY(update_columns(k0, ncols, 0, M2, 0));
       }
     } else if constexpr (std::is_same<T, double2>::value) {
       // FP64 path: the trailing update C -= A B on the FP64 tensor cores (zgemm_f64.cu)
@@ -792,12 +849,6 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   };
   auto pk = panel_kernel<T, NB, NT>;
   auto pkc = panel_reg_kernel<T, NB>;
-  // the largest rows per CTA of a cluster panel (shared memory of the opt-in limit, less the
-  // static arrays)
-  int rpc_max_c = 0;
-  const size_t static_c = (sizeof(T) == sizeof(double2) ? 20 : 12) * 1024;
-  while (rpc_max_c < kRegPanelRows && panel_reg_smem<T, NB>(rpc_max_c + 1) + static_c <= (size_t)c->smem_optin)
-    ++rpc_max_c;
   auto cluster_fits = [&](int g) -> bool {  // can the GPU hold a cluster of g such CTAs
     signed char& ok = c->cluster_ok[sizeof(T) == sizeof(double2)][g];
     if (ok == 0) {
@@ -823,10 +874,32 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     }
     return ok == 1;
   };
+  const int sub_rows = 16 * kSubThreads * (sizeof(T) == sizeof(double2) ? 2 : 4);
+  auto tall_fits = [&](int m) -> bool {  // sub-panels on one 16-CTA cluster
+    return NB >= 2 * kSubW && m <= sub_rows && panel_sub_smem<T>((m + 15) / 16) + 16 * 1024 <= (size_t)c->smem_optin &&
+           cluster_fits(16);
+  };
+  if constexpr (sizeof(T) == sizeof(float2)) {
+    if (mixed && c->panel_cluster && c->lookahead > 0 && N - NB >= c->lookahead && c->nsm > 32 && cluster_fits(16)) {
+      if (!c->side) {
+        int least = 0, greatest = 0;
+        HPR_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        HPR_CUDA_TRY(cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, greatest));
+      }
+      for (cudaEvent_t& e : c->side_ev)
+        if (!e) HPR_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      ahead_fits = [&](int k1) {
+        const int m1 = N - k1;
+        return m1 > NB && m1 >= c->lookahead && ((rpc_max_c > 0 && m1 <= 16 * rpc_max_c) || tall_fits(m1));
+      };
+    }
+  }
   for (int s = 0; s < nsteps; ++s) {
     const int k0 = s * NB;
     const int ncols = std::min(NB, N - k0);
     const int m = N - k0;
+    const bool ahead = ahead_k0 >= 0;  // this panel runs beside the update of the step before
+    const cudaStream_t ps = ahead ? c->side : c->stream;
     if (c->panel_cluster && rpc_max_c > 0 && m <= 16 * rpc_max_c) {
       // the whole panel in one cluster: as many CTAs as panel_rpc_min rows allow, at most 16
       // (one CTA up to 128 rows: without the cluster's exchange a column is shorter)
@@ -864,19 +937,24 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
         cfg.gridDim = dim3(Gc);
         cfg.blockDim = dim3(kRegPanelThreads);
         cfg.dynamicSmemBytes = smc;
-        cfg.stream = c->stream;
-        cudaLaunchAttribute at[1];
+        cfg.stream = ps;
+        cudaLaunchAttribute at[2];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = Gc;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
+        at[1].id = cudaLaunchAttributeLaunchCompletionEvent;
+        at[1].val.launchCompletionEvent.event = c->side_ev[1];
+        at[1].val.launchCompletionEvent.flags = 0;
         cfg.attrs = at;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = ahead ? 2 : 1;
         const cudaError_t e = cudaLaunchKernelEx(&cfg, pkc, pa);
         if (e != cudaSuccess)
           return fail(HPRMAT_B200_ERR_CUDA, "cluster panel launch (step %d, %d CTAs of %d rows, %zu B shared): %s", s,
                       Gc, rpcc, smc, cudaGetErrorString(e));
         ++c->launches;
+        if (ahead) TRY(ahead_update());
+        TRY(ahead_join());
         if (k0 + ncols >= N) break;
         TRY(after_step(s, k0, ncols, pa.sw));
         continue;
@@ -884,12 +962,9 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     }
     if constexpr (NB >= 2 * kSubW) {
       // a tall panel: sub-panels on one 16-CTA cluster, the rest of the panel on all SMs
-      const int rpt_max = sizeof(T) == sizeof(double2) ? 2 : 4;
       const int rps = (m + 15) / 16;
       const size_t ssm = panel_sub_smem<T>(rps);
-      const size_t sstatic = 16 * 1024;
-      if (c->panel_cluster && rps <= rpt_max * kSubThreads && ssm + sstatic <= (size_t)c->smem_optin &&
-          cluster_fits(16)) {
+      if (c->panel_cluster && tall_fits(m)) {
         TRY(c->ppos.ensure((size_t)(N + NB) * sizeof(int)));
         SubArgs<T> sa;
         sa.W = W;
@@ -918,17 +993,20 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
           cfg.gridDim = dim3(16);
           cfg.blockDim = dim3(kSubThreads);
           cfg.dynamicSmemBytes = ssm;
-          cfg.stream = c->stream;
-          cudaLaunchAttribute at[1];
+          cfg.stream = ps;
+          cudaLaunchAttribute at[2];
           at[0].id = cudaLaunchAttributeClusterDimension;
           at[0].val.clusterDim.x = 16;
           at[0].val.clusterDim.y = 1;
           at[0].val.clusterDim.z = 1;
+          at[1].id = cudaLaunchAttributeLaunchCompletionEvent;
+          at[1].val.launchCompletionEvent.event = c->side_ev[1];
+          at[1].val.launchCompletionEvent.flags = 0;
           cfg.attrs = at;
-          cfg.numAttrs = 1;
+          cfg.numAttrs = ahead && sa.c0 == 0 ? 2 : 1;
           HPR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, sa));
           ++c->launches;
-          return HPRMAT_B200_OK;
+          return ahead && sa.c0 == 0 ? ahead_update() : HPRMAT_B200_OK;
         };
         const int rpt = (rps + kSubThreads - 1) / kSubThreads;
         for (sa.c0 = 0; sa.c0 < ncols; sa.c0 += kSubW) {
@@ -936,22 +1014,27 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
           else if (rpt == 2) TRY(sub(panel_sub_kernel<T, 2>));
           else if constexpr (sizeof(T) == sizeof(float2)) TRY(rpt == 3 ? sub(panel_sub_kernel<T, 3>) : sub(panel_sub_kernel<T, 4>));
           if (sa.c0 + kSubW < ncols) {
-            panel_rest_kernel<T, NB><<<cdiv_u(m, kRestRows), 256, 0, c->stream>>>(sa);
+            panel_rest_kernel<T, NB><<<cdiv_u(m, kRestRows), 256, 0, ps>>>(sa);
             LAUNCH_CHECK();
           }
         }
         if constexpr (sizeof(T) == sizeof(float2)) {
           if (sa.lup) {
-            panel_planes_kernel<NB><<<cdiv_u(m, 32), 256, 0, c->stream>>>(sa);
+            panel_planes_kernel<NB><<<cdiv_u(m, 32), 256, 0, ps>>>(sa);
             LAUNCH_CHECK();
           }
         }
-        panel_place_kernel<T, NB><<<cdiv_u(ncols, kPlaceCols), 256, 0, c->stream>>>(sa);
+        panel_place_kernel<T, NB><<<cdiv_u(ncols, kPlaceCols), 256, 0, ps>>>(sa);
         LAUNCH_CHECK();
+        TRY(ahead_join());
         if (k0 + ncols >= N) break;
         TRY(after_step(s, k0, ncols, sa.sw));
         continue;
       }
+    }
+    if (ahead) {  // no cluster panel after all
+      TRY(update_columns(ahead_k0, NB, NB, N - ahead_k0 - NB, 0));
+      ahead_k0 = -1;
     }
     // CTAs of the panel: at least panel_rpc_min rows each (fewer CTAs contend less for the
     // per-column barrier), as many as the shared memory needs
@@ -2397,6 +2480,12 @@ int hprmat_b200_destroy(hprmat_b200_ctx* c) {
   if (!c) return HPRMAT_B200_OK;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
+  if (c->side) {
+    cudaStreamSynchronize(c->side);
+    cudaStreamDestroy(c->side);
+  }
+  for (cudaEvent_t e : c->side_ev)
+    if (e) cudaEventDestroy(e);
   DevBuf* bufs[] = {&c->mesh, &c->W, &c->A64, &c->X, &c->X64, &c->R64, &c->B64, &c->V, &c->Z, &c->gm,
                     &c->swaps, &c->ipiv, &c->stage, &c->status, &c->ops, &c->inv, &c->chan, &c->rmat,
                     &c->zwork, &c->cpot, &c->cu, &c->lup, &c->rop, &c->rsurf, &c->vt, &c->rlo,
@@ -4207,6 +4296,11 @@ int hprmat_b200_dev_set_tuning(hprmat_b200_ctx* c, const char* key, int value) {
   }
   if (strcmp(key, "f64_pair") == 0) {
     c->f64_pair = value != 0;
+    return HPRMAT_B200_OK;
+  }
+  if (strcmp(key, "lookahead") == 0) {  // fewest trailing rows for the LU's look-ahead (0: never)
+    if (value < 0) return fail(HPRMAT_B200_ERR_ARG, "lookahead must be >= 0");
+    c->lookahead = value;
     return HPRMAT_B200_OK;
   }
   if (strcmp(key, "hess_workers") == 0) {  // shifted scan: blocks in flight at once, 1..8

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+from hprmat_b200 import _native as nat
 from hprmat_b200 import api
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,33 @@ def test_tall_panels(precision, n):
     del a, at
     torch.cuda.empty_cache()  # the largest sizes' memory back for the tests that follow
     assert r <= bound
+
+
+@pytest.mark.parametrize("n", [257, 385, 1025, 2995, 3333, 6400])
+def test_lookahead_leaves_the_factors_alone(n):
+    """A trailing matrix updated beside the next panel (from 129 rows on, the default, never): the same
+    solution bit for bit, as every element sees the same operations."""
+    rng = np.random.default_rng(n)
+    a = rng.uniform(-1, 1, (n, n)) + 1j * rng.uniform(-1, 1, (n, n))
+    b = rng.uniform(-1, 1, (n, 2)) + 0j
+    lib = nat.load()
+    xs = []
+    with api.Context(precision="mixed", max_refine=8) as ctx:
+        for rows in (0, 129, 2048, 129):
+            nat.check(lib.hprmat_b200_dev_set_tuning(ctx._h, b"lookahead", rows))
+            xs.append(ctx.solve_linear(a, b, allow_unconverged=True))
+    for x in xs[1:]:
+        assert np.array_equal(x, xs[0])
+
+
+@pytest.mark.parametrize("precision,nb", [("fp64", 16), ("fp64", 32), ("fp64", 64), ("mixed", 16), ("mixed", 32),
+                                          ("mixed", 64), ("mixed", 128)])
+def test_block_sizes(precision, nb):
+    """U12's substitution at every block size, with ragged last blocks and column tails: the bound of
+    the first test."""
+    for n in (nb + 1, 2 * nb - 1, 3 * nb + 33, 4 * nb + 64):
+        a = _matrix(n, False)
+        b = np.random.default_rng(n).uniform(-1, 1, (n, 2)) + 0j
+        with api.Context(precision=precision, max_refine=8, tol=1e-15, panel_nb=nb) as ctx:
+            x = ctx.solve_linear(a, b, allow_unconverged=True)
+        assert np.abs(a @ x - b).max() <= 8 * n * 2.0 ** -53 * np.abs(a).sum(1).max() * np.abs(x).max()
