@@ -616,8 +616,8 @@ __global__ void wait_probe_kernel(int* counter, int* timeout_flag, unsigned limi
 // C[M x N] -= A[M x K] B[K x N] in complex FP64 (column-major) on the context's stream, by
 // this library's DMMA kernel (zgemm_f64.cu).
 static int zgemm_update(hprmat_b200_ctx* c, int M, int N, int K, const double2* A, long lda, const double2* B,
-                        long ldb, double2* C, long ldc) {
-  if (zgemm_f64_update(M, N, K, A, lda, B, ldb, C, ldc, c->stream))
+                        long ldb, double2* C, long ldc, int max_sms = 0) {
+  if (zgemm_f64_update(M, N, K, A, lda, B, ldb, C, ldc, c->stream, max_sms))
     return fail(HPRMAT_B200_ERR_CUDA, "FP64 complex GEMM update: %s", hprmat_b200_last_error());
   ++c->launches;
   return HPRMAT_B200_OK;
@@ -709,15 +709,18 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   const size_t static_c = (sizeof(T) == sizeof(double2) ? 20 : 12) * 1024;
   while (rpc_max_c < kRegPanelRows && panel_reg_smem<T, NB>(rpc_max_c + 1) + static_c <= (size_t)c->smem_optin)
     ++rpc_max_c;
-  // Look-ahead of the mixed path: the panel of step s + 1 needs only its own columns of step s's
+  // Look-ahead: the panel of step s + 1 needs only its own columns of step s's
   // trailing update.  They are updated first; the panel then runs on a stream of its own, on the 16
   // SMs of its cluster, and the update of the other columns beside it on the rest.  The update
   // starts when the panel's first cluster is resident (a launch completion event: persistent CTAs
   // placed first would leave no GPC with 16 free SMs), and the next step waits for both.
   // Measured (factorisation alone, without -> with): N = 3000 6.89 -> 6.74 ms, 6400 21.5 -> 19.1, 12800 69.6
   // -> 56.9, 25600 330 -> 303.  The line at 2048 rows: 1000 to 3000 measure alike (the panel hides 15 to
-  // 45 us of update there and pays 12 for the launch of its columns).  The same factors bit for bit.
-  int ahead_k0 = -1;  // step whose other columns are still to be updated
+  // 45 us of update there and pays 12 for the launch of its columns).  The same factors bit for bit
+  // (FP64: to rounding, as the GEMM splits K by its number of tiles).
+  // The FP64 pairs of block steps do the same after their second panel, from a quarter of those rows on:
+  // N = 1000 2.73 -> 2.69 ms, 2000 6.21 -> 5.62, 4000 17.9 -> 15.9, 9600 115.0 -> 112.3.
+  std::function<int()> ahead_rest;  // the update of the other columns, while it is still to be launched
   // trailing update of the columns j0 .. j1 right of the panel at k0, on at most max_grid CTAs (0: all)
   auto update_columns = [&](int k0, int ncols, int j0, int j1, int max_grid) -> int {
     const int k1 = k0 + ncols, M2 = N - k1;
@@ -750,14 +753,20 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     while (r < most && 6.5e-4 * rows * rows / (c->nsm - r) < subs + 0.91 * rows / r) r += 4;
     return r;
   };
+  auto ahead_start = [&](std::function<int()> rest) -> int {  // the next panel's columns are up to date
+    HPR_CUDA_TRY(cudaEventRecord(c->side_ev[0], c->stream));
+    HPR_CUDA_TRY(cudaStreamWaitEvent(c->side, c->side_ev[0], 0));
+    ahead_rest = std::move(rest);
+    return HPRMAT_B200_OK;
+  };
   // after the first kernel of the panel beside which the update runs (launched with side_ev[1])
   auto ahead_update = [&]() -> int {
     HPR_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->side_ev[1], 0));
-    return update_columns(ahead_k0, NB, NB, N - ahead_k0 - NB, c->nsm - ahead_sms(N - ahead_k0 - NB));
+    return ahead_rest();
   };
   auto ahead_join = [&]() -> int {  // after the panel's last kernel
-    if (ahead_k0 < 0) return HPRMAT_B200_OK;
-    ahead_k0 = -1;
+    if (!ahead_rest) return HPRMAT_B200_OK;
+    ahead_rest = nullptr;
     HPR_CUDA_TRY(cudaEventRecord(c->side_ev[2], c->side));
     HPR_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->side_ev[2], 0));
     return HPRMAT_B200_OK;
@@ -773,9 +782,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     if (mixed) {
       if (ahead_fits(k0 + ncols)) {  // now the next panel's columns only, the others beside that panel
         TRY(update_columns(k0, ncols, 0, NB, 0));
-        HPR_CUDA_TRY(cudaEventRecord(c->side_ev[0], c->stream));
-        HPR_CUDA_TRY(cudaStreamWaitEvent(c->side, c->side_ev[0], 0));
-        ahead_k0 = k0;
+        TRY(ahead_start([&, k0, M2]() { return update_columns(k0, NB, NB, M2, c->nsm - ahead_sms(M2)); }));
       } else {
         TRY(update_columns(k0, ncols, 0, M2, 0));
       }
@@ -837,7 +844,16 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
       LAUNCH_CHECK();
       patch_rows_kernel<T><<<1, 256, 0, c->stream>>>(W, ld, s1.extra_dst, s1.extra_src, s1.n_extra, k2, k0, NB, LL, m2);
       LAUNCH_CHECK();
-      TRY(zgemm_update(c, m2, m2, 2 * NB, LL, m2, W + k0 + (size_t)k2 * ld, ld, W + k2 + (size_t)k2 * ld, ld));
+      auto update = [&, k0, k2, m2, LL](int j0, int j1, int max_sms) {
+        return zgemm_update(c, m2, j1 - j0, 2 * NB, LL, m2, W + k0 + (size_t)(k2 + j0) * ld, ld,
+                            W + k2 + (size_t)(k2 + j0) * ld, ld, max_sms);
+      };
+      if (ahead_fits(k2)) {
+        TRY(update(0, NB, 0));
+        TRY(ahead_start([&, update, m2]() { return update(NB, m2, c->nsm - 16); }));
+      } else {
+        TRY(update(0, m2, 0));
+      }
     }
     return HPRMAT_B200_OK;
   };
@@ -879,26 +895,28 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     return NB >= 2 * kSubW && m <= sub_rows && panel_sub_smem<T>((m + 15) / 16) + 16 * 1024 <= (size_t)c->smem_optin &&
            cluster_fits(16);
   };
-  if constexpr (sizeof(T) == sizeof(float2)) {
-    if (mixed && c->panel_cluster && c->lookahead > 0 && N - NB >= c->lookahead && c->nsm > 32 && cluster_fits(16)) {
-      if (!c->side) {
-        int least = 0, greatest = 0;
-        HPR_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        HPR_CUDA_TRY(cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, greatest));
-      }
-      for (cudaEvent_t& e : c->side_ev)
-        if (!e) HPR_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      ahead_fits = [&](int k1) {
-        const int m1 = N - k1;
-        return m1 > NB && m1 >= c->lookahead && ((rpc_max_c > 0 && m1 <= 16 * rpc_max_c) || tall_fits(m1));
-      };
+  const int ahead_min = mixed ? c->lookahead : c->lookahead / 4;
+  if ((mixed || pair) && c->panel_cluster && ahead_min > 0 && N - NB >= ahead_min && c->nsm > 32 && cluster_fits(16)) {
+    if (!c->side) {
+      int least = 0, greatest = 0;
+      HPR_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+      HPR_CUDA_TRY(cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, greatest));
     }
+    for (cudaEvent_t& e : c->side_ev)
+      if (!e) HPR_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    ahead_fits = [&](int k1) {
+      // and while 16 SMs cost the update of m rows less than the panel takes: measured times of both
+      const int m1 = N - k1;
+      const double m = m1, upd = (mixed ? 4.4e-6 : 2.8e-5) * m * m, panel = mixed ? 200.0 + 0.016 * m : 120.0 + 0.01 * m;
+      return m1 > NB && m1 >= ahead_min && upd * 16.0 / (c->nsm - 16) < panel &&
+             ((rpc_max_c > 0 && m1 <= 16 * rpc_max_c) || tall_fits(m1));
+    };
   }
   for (int s = 0; s < nsteps; ++s) {
     const int k0 = s * NB;
     const int ncols = std::min(NB, N - k0);
     const int m = N - k0;
-    const bool ahead = ahead_k0 >= 0;  // this panel runs beside the update of the step before
+    const bool ahead = (bool)ahead_rest;  // this panel runs beside the update of the step before
     const cudaStream_t ps = ahead ? c->side : c->stream;
     if (c->panel_cluster && rpc_max_c > 0 && m <= 16 * rpc_max_c) {
       // the whole panel in one cluster: as many CTAs as panel_rpc_min rows allow, at most 16
@@ -1033,8 +1051,8 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
       }
     }
     if (ahead) {  // no cluster panel after all
-      TRY(update_columns(ahead_k0, NB, NB, N - ahead_k0 - NB, 0));
-      ahead_k0 = -1;
+      TRY(ahead_rest());
+      ahead_rest = nullptr;
     }
     // CTAs of the panel: at least panel_rpc_min rows each (fewer CTAs contend less for the
     // per-column barrier), as many as the shared memory needs

@@ -315,12 +315,12 @@ int launch_zgemm(long grid, int M, int N, int K, const double2* A, long lda, con
 }  // namespace
 
 int zgemm_f64_update(int M, int N, int K, const double2* A, long lda, const double2* B, long ldb, double2* C,
-                     long ldc, cudaStream_t s) {
-  return zgemm_f64_update_batched(M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, s);
+                     long ldc, cudaStream_t s, int max_sms) {
+  return zgemm_f64_update_batched(M, N, K, A, lda, 0, B, ldb, 0, C, ldc, 0, 1, s, max_sms);
 }
 
 int zgemm_f64_update_batched(int M, int N, int K, const double2* A, long lda, long sA, const double2* B, long ldb,
-                             long sB, double2* C, long ldc, long sC, int batch, cudaStream_t s) {
+                             long sB, double2* C, long ldc, long sC, int batch, cudaStream_t s, int max_sms) {
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return 0;
   if (((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)C & 15) || lda < M || ldb < K || ldc < M || sA < 0 ||
       sB < 0 || sC < 0) {
@@ -336,6 +336,7 @@ int zgemm_f64_update_batched(int M, int N, int K, const double2* A, long lda, lo
   int dev = 0, nsm = 0;
   HPR_CUDA_TRY(cudaGetDevice(&dev));
   HPR_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  if (max_sms > 0 && max_sms < nsm) nsm = max_sms;
   const long ntiles = (long)((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN) * batch;
   const long slots = 2L * nsm;  // two resident CTAs per SM
   // Few tiles, long K: split K over a cluster while all CTAs fit at once and each keeps 4 chunks or

@@ -74,8 +74,8 @@ int hprmat_b200_dev_counters(hprmat_b200_ctx* ctx, unsigned long long* launches,
                       time (0);
      "hess_cluster"   CTAs of the blocked reduction's column-step cluster: 8, 16, or 0 to
                       take 16 where the GPU holds such a cluster;
-     "lookahead"      mixed LU: fewest rows of a trailing matrix that is updated beside the next
-                      panel (default 2048; 0: never);
+     "lookahead"      LU: fewest rows of a trailing matrix that is updated beside the next panel
+                      (default 2048, a quarter of it for FP64; 0: never);
      "hess_workers"   shifted scan: J-pi blocks in flight at once, each on a worker context
                       of its own, 1..8 (3). */
 int hprmat_b200_dev_set_tuning(hprmat_b200_ctx* ctx, const char* key, int value);

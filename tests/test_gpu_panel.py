@@ -92,3 +92,18 @@ def test_block_sizes(precision, nb):
         with api.Context(precision=precision, max_refine=8, tol=1e-15, panel_nb=nb) as ctx:
             x = ctx.solve_linear(a, b, allow_unconverged=True)
         assert np.abs(a @ x - b).max() <= 8 * n * 2.0 ** -53 * np.abs(a).sum(1).max() * np.abs(x).max()
+
+
+@pytest.mark.parametrize("n", [193, 257, 385, 1025, 3333])
+def test_fp64_lookahead(n):
+    """The FP64 LU's pairs of block steps (look-ahead from 65 rows on, the default): the first test's bound,
+    and the same bits from a second run."""
+    a, lib = _matrix(n, False), nat.load()
+    b = np.random.default_rng(n).uniform(-1, 1, (n, 2)) + 0j
+    xs = {}
+    with api.Context(precision="fp64") as ctx:
+        for rows in (260, 2048, 260, 2048):
+            nat.check(lib.hprmat_b200_dev_set_tuning(ctx._h, b"lookahead", rows))
+            x = ctx.solve_linear(a, b)
+            assert np.abs(a @ x - b).max() <= 8 * n * 2.0 ** -53 * np.abs(a).sum(1).max() * np.abs(x).max()
+            assert np.array_equal(xs.setdefault(rows, x), x)
