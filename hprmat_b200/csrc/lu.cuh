@@ -363,15 +363,16 @@ struct TrsmArgs {
   int mode;          // 0: interchanges and solve; 1: interchanges only; 2: solve only (rows k0..)
 };
 
-// Interchanges and substitution with the right-hand sides in registers: LN = NB / 16 lanes share a column, lane g
-// holding rows LN a + g in x[a], a < 16.  A step broadcasts x_k within the lanes of a column and
-// updates the rows below; L11 is staged in shared memory once per CTA, and a group of 2 NB threads
-// walks over blocks of 32 columns (no barrier between the steps).  x moves one register down every LN steps and its end takes the
-// finished row, so that the code of LN steps serves several blocks of them and the rows are back in
-// place after 16; the displaced rows travel through the same shared memory meanwhile.
-// Measured, average over the steps: FP64, N = 4000 with NB = 64, against one barrier and one L2 read of L's column
-// per step: 41 -> 12 us.  Mixed, NB = 128, against
-// the inverse of L11, a row gather, a tensor-core product and a split of its result as four launches:
+// Interchanges and substitution with the right-hand sides in registers: LN = NB / 16 lanes share a
+// column, lane g holding rows LN a + g in x[a], a < 16.  A step broadcasts x_k within the lanes of a
+// column and updates the rows below; L11 is staged in shared memory once per CTA, and a group of 2 NB
+// threads walks over blocks of 32 columns (no barrier between the steps).  x moves one register down
+// every LN steps and its end takes the finished row, so that the code of LN steps serves several
+// blocks of them and the rows are back in place after 16; the displaced rows travel through the same
+// shared memory meanwhile.
+// Measured, average over the steps: FP64, N = 4000 with NB = 64, against one barrier and one L2 read
+// of L's column per step: 41 -> 12 us.  Mixed, NB = 128, against the inverse of L11, a row gather, a
+// tensor-core product and a split of its result as four launches:
 // N = 400 40 -> 22 us, N = 3000 46 -> 23, N = 6400 48 -> 27, N = 25600 66 -> 71 (0.3 % of that
 // factorisation); and no inverse enters U any more.  Bound by the chain of NB broadcasts and updates,
 // in the wide case by the traffic of U12's three copies.

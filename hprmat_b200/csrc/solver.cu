@@ -501,8 +501,8 @@ static int wave_prepare(hprmat_b200_ctx* c, const LUState& st) {
 
 // Orders whose solves use explicit inverses of the whole factors (tri_solve.cuh): up to
 // kInvMaxSteps blocks of 128.  Whole rmatrix calls (seeded production potentials), wavefront
-// against inverses: N = 400 1.92 / 1.49 ms, 720 2.95 / 2.35, 992 3.71 / 3.16, 1240 4.65 / 4.04,
-// 1743 6.18 / 6.21, 1980 8.89 / 8.92: the inverses' N^3 passes what the sweeps cost near 14 blocks.
+// against inverses: N = 200 1.00 / 0.76 ms, 400 1.73 / 1.32, 600 2.69 / 2.03, 720 2.47 / 2.21, 992 3.11 /
+// 2.85, 1240 3.94 / 3.91: the inverses' N^3 passes what the sweeps cost at 10 blocks.
 // Refinement iterations are the same on both sides.
 constexpr int kInvMaxSteps = 10;
 
@@ -699,9 +699,9 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
       const int groups = NB == 128 && blocks > ctas ? 2 : 1;
       TRY(set_smem(tk, trsm_smem<T, NB>(groups)));
       tk<<<std::min(cdiv_u(blocks, groups), ctas), groups * trsm_threads<NB>(), trsm_smem<T, NB>(groups), c->stream>>>(ta);
+      LAUNCH_CHECK();
+      return HPRMAT_B200_OK;
     }
-    LAUNCH_CHECK();
-    return HPRMAT_B200_OK;
   };
   // the largest rows per CTA of a cluster panel (shared memory of the opt-in limit, less the
   // static arrays)
@@ -1588,15 +1588,16 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
     gmres_start_kernel<256><<<nrhs, 256, 0, c->stream>>>(gs);
     LAUNCH_CHECK();
     // the first cycle starts from the FP32 solution; a later cycle aims at what is left to
-    // the tolerance (a tenth of tol / rel), so that one polishing cycle usually ends it; with the
-    // surface rule also at what that rule will ask of it (1e3 change est < surface_tol, the change in
-    // R being up to about half of rel).  At N = 6400 that ends 7 of 8 potentials after two cycles, 3 of
-    // 8 without it (35.7 against 37.5 ms in the mean); at N = 25600 it changes nothing.  Scaling the
+    // the tolerance (a tenth of tol / rel), so that one polishing cycle usually ends it; the second
+    // one with the surface rule also at what that rule will ask of it (1e3 change est < surface_tol,
+    // the change in R being up to about half of rel).  At N = 6400 that ends 7 of 8 potentials after
+    // two cycles, 3 of 8 without it (35.7 against 37.5 ms in the mean); iterations of 14 potentials at N =
+    // 25600 and 12800: 203 without it, 200 with it, 204 with it in every later cycle.  Scaling the
     // aim by the last change in R instead asked for more iterations without saving cycles.
     double inner_tol = c->inner_tol0;
     if (outer > 0) {
       double aim = 0.1 * c->opts.tol;
-      if (surf && c->opts.surface_tol > 0.0) aim = std::min(aim, 2e-3 * c->opts.surface_tol);
+      if (surf && outer == 1 && c->opts.surface_tol > 0.0) aim = std::min(aim, 2e-3 * c->opts.surface_tol);
       inner_tol = std::min(1e-2, std::max(1e-8, aim / std::max(rel, 1e-300)));
     }
     int jdone = 0;
@@ -2485,6 +2486,7 @@ int hprmat_b200_create(int device, const hprmat_b200_opts* opts, hprmat_b200_ctx
     return s;
   }
   HPR_CUDA_TRY(cudaMemset(c->status.p, 0, 64 * sizeof(int)));
+  c->tcplan.h_err = c->h_status + 63;  // beyond the status words' copy (kStatusCopy)
   s = tc_gemm_init(c->tcplan, device);
   if (s != HPRMAT_B200_OK) {
     delete c;
@@ -2515,7 +2517,6 @@ int hprmat_b200_destroy(hprmat_b200_ctx* c) {
   for (cudaEvent_t e : c->ev) cudaEventDestroy(e);
   if (c->h_status) cudaFreeHost(c->h_status);
   if (c->h_norms) cudaFreeHost(c->h_norms);
-  if (c->tcplan.h_err) cudaFreeHost(c->tcplan.h_err);
   if (c->tcplan.d_err) cudaFree(c->tcplan.d_err);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;

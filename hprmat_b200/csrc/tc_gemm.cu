@@ -277,7 +277,6 @@ int tc_gemm_init(TcGemmPlan& p, int device) {
   if (!p.d_err) {
     HPR_CUDA_TRY(cudaMalloc(&p.d_err, sizeof(int)));
     HPR_CUDA_TRY(cudaMemset(p.d_err, 0, sizeof(int)));
-    HPR_CUDA_TRY(cudaMallocHost(&p.h_err, sizeof(int)));
   }
   HPR_CUDA_TRY(cudaFuncSetAttribute(tc_update_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     TileCfg<256>::kSmemBytes));

@@ -12,7 +12,7 @@ struct TcGemmPlan {
   int nsm = 0;
   void* encode = nullptr;  // cuTensorMapEncodeTiled, fetched through the runtime
   int* d_err = nullptr;    // device word: nonzero if a bounded wait gave up
-  int* h_err = nullptr;    // its pinned copy (tc_gemm_check_async)
+  int* h_err = nullptr;    // its pinned copy (tc_gemm_check_async), memory of the plan's owner
   int max_grid = 0;        // most CTAs of a persistent update (0: one per SM); concurrent
                            // solves (scan workers) leave SMs to each other with a smaller grid
 };
