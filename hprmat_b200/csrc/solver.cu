@@ -634,6 +634,10 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   st.nb = NB;
   st.nsteps = nsteps;
   int* status = c->status.as<int>();
+  if (c->side) {  // a factorisation that ended in an error may have left its panel there
+    HPR_CUDA_TRY(cudaEventRecord(c->side_ev[2], c->side));
+    HPR_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->side_ev[2], 0));
+  }
   HPR_CUDA_TRY(cudaMemsetAsync(status, 0, SW_COUNT * sizeof(int), c->stream));
   const int G0 = std::min(c->nsm, std::max(1, (N + 31) / 32));
   TRY(c->stage.ensure((size_t)2 * G0 * NB * sizeof(T) + (size_t)NB * sizeof(unsigned long long) +
@@ -897,13 +901,13 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   };
   const int ahead_min = mixed ? c->lookahead : c->lookahead / 4;
   if ((mixed || pair) && c->panel_cluster && ahead_min > 0 && N - NB >= ahead_min && c->nsm > 32 && cluster_fits(16)) {
+    for (cudaEvent_t& e : c->side_ev)
+      if (!e) HPR_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     if (!c->side) {
       int least = 0, greatest = 0;
       HPR_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
       HPR_CUDA_TRY(cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, greatest));
     }
-    for (cudaEvent_t& e : c->side_ev)
-      if (!e) HPR_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     ahead_fits = [&](int k1) {
       // and while 16 SMs cost the update of m rows less than the panel takes: measured times of both
       const int m1 = N - k1;
