@@ -1441,10 +1441,25 @@ static int frob_norm(hprmat_b200_ctx* c, const double2* X, long ldx, int N, int 
   return HPRMAT_B200_OK;
 }
 
+// Waits for the stream.  mixed: also that no wait of a tensor-core solve queued so far gave up, which
+// would invalidate its result.
+static int sync_solves(hprmat_b200_ctx* c, bool mixed) {
+  if (mixed && tc_gemm_check_async(c->tcplan, c->stream))
+    return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
+  HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  if (mixed) {
+    int err = 0;
+    TRY(tc_gemm_check_done(c->tcplan, c->stream, &err));
+    if (err) return fail(HPRMAT_B200_ERR_TIMEOUT, "tensor-core solve: wait limit exceeded at site %d", err);
+  }
+  return HPRMAT_B200_OK;
+}
+
 // Mixed path: X64 (N x nrhs, FP64) from the FP32 factors, refined with FGMRES on the FP64
 // operator.  Each outer step: r = B - C X; stop when |r|_F/|B|_F < tol; otherwise run
 // up to gmres_m flexible-GMRES iterations on C d = r, preconditioned by the FP32 LU solve, and
 // X += d.  Returns NOT_CONVERGED if max_refine outer corrections did not reach tol.
+// Its last solve may still be queued when it returns: the caller's next wait is sync_solves.
 static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W32, const LUState& st,
                         double2* X64, long ldx, int nrhs, double bnorm, double cnorm, hprmat_b200_stats* stats,
                         int max_outer = -1, bool error_based = false) {
@@ -1533,14 +1548,7 @@ static int refine_mixed(hprmat_b200_ctx* c, const Operator& op, const float2* W3
       colnorm2_kernel<<<nrhs, 256, 0, c->stream>>>(V + vstride, ldv, N, h_scale);
       LAUNCH_CHECK();
     }
-    if (tc_gemm_check_async(c->tcplan, c->stream)) return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
-    HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    {
-      // a bounded wait that gave up inside a tensor-core solve invalidates the result
-      int err = 0;
-      TRY(tc_gemm_check_done(c->tcplan, c->stream, &err));
-      if (err) return fail(HPRMAT_B200_ERR_TIMEOUT, "tensor-core solve: wait limit exceeded at site %d", err);
-    }
+    TRY(sync_solves(c, true));
     const double rel = norm_of(h_res) / bnorm;
     if (outer == 0) rel0 = rel;
     double change = -1.0;
@@ -2092,7 +2100,7 @@ static int rmatrix_core(hprmat_b200_ctx* c, int nch, const int* lval, const doub
                                                 wf ? c->wfz.as<double2>() + (size_t)is * nn : zo + nn, d_info);
     LAUNCH_CHECK();
     HPR_CUDA_TRY(cudaMemcpyAsync(c->h_status, c->status.p, SW_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    TRY(sync_solves(c, mixed));
     if (c->h_status[SW_INFO] != 0)
       return fail(HPRMAT_B200_SINGULAR, "singular R00 + rmax1 R in the propagation to interval %d", is + 1);
   }
@@ -2104,14 +2112,7 @@ static int rmatrix_core(hprmat_b200_ctx* c, int nch, const int* lval, const doub
                                             zo + std::max(1, no * no), d_cu, ndim, d_info);
   LAUNCH_CHECK();
   HPR_CUDA_TRY(cudaMemcpyAsync(c->h_status, c->status.p, SW_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  if (mixed && tc_gemm_check_async(c->tcplan, c->stream))
-    return fail(HPRMAT_B200_ERR_CUDA, "%s", hprmat_b200_last_error());
-  HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  if (mixed) {  // the refinement's last solve (after its own last check)
-    int err = 0;
-    TRY(tc_gemm_check_done(c->tcplan, c->stream, &err));
-    if (err) return fail(HPRMAT_B200_ERR_TIMEOUT, "tensor-core solve: wait limit exceeded at site %d", err);
-  }
+  TRY(sync_solves(c, mixed));
   if (c->h_status[SW_INFO] != 0) return fail(HPRMAT_B200_SINGULAR, "singular Z_O in the collision-matrix step");
   if (wf) {
     // surface amplitudes from U, carried inwards, then the wave function per interval
@@ -2377,7 +2378,7 @@ static int solve_dense_core(hprmat_b200_ctx* c, const double2* dA, double2* dB, 
     if (status != HPRMAT_B200_OK && status != HPRMAT_B200_NOT_CONVERGED) return status;
     copy_d_kernel<<<gr, 256, 0, c->stream>>>(X64, ld, dB, N, N);
     LAUNCH_CHECK();
-    HPR_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    TRY(sync_solves(c, true));
     if (stats) stats->ms_refine = ms_since(t3);
   }
   if (!mixed || fallback) {
