@@ -62,6 +62,13 @@ constexpr int kPanelTraceW = 5 + 160;
 // that orders over the element type's whole range (FP64 panels: magnitudes far outside the
 // float range too), with the lowest row winning among equal moduli.
 
+// The interchange list and pivots of a panel that gave up (a bounded wait ran out): no row moves, so
+// that the kernels behind it in the stream find valid rows until the host reads SW_TIMEOUT.
+__device__ __forceinline__ void no_interchanges(const StepSwaps& sw, int* ipiv, int k0, int ncols, int tid, int nthreads) {
+  for (int j = tid; j < ncols; j += nthreads) sw.top_src[j] = ipiv[k0 + j] = k0 + j;
+  if (tid == 0) *sw.n_extra = 0;
+}
+
 // End of a panel factorisation: the CTA's factored rows back into W, its L21 rows into the LU planes (mixed path), and from CTA 0 the pivots, the growth
 // and the step's row-interchange list.
 template <typename T, int NB, int NT>

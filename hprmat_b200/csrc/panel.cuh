@@ -49,6 +49,22 @@ __host__ __device__ constexpr size_t panel_reg_smem(int rpc) {
   return ((size_t)NB * (size_t)(rpc | 1) + (NB - W) * W + 2) * sizeof(T);
 }
 
+// A wait that runs out: the thread sets SW_TIMEOUT, waits for no message any more and goes through the
+// remaining columns with whatever the buffers hold, so that every CTA still meets the others at the cluster's
+// barriers.  Positions may then be any integers, and rows may share one.  So SW_TIMEOUT is read again after
+// the last barrier, behind which every CTA sees the same value, before anything that goes by a position is
+// written; a panel that gave up leaves no_interchanges.
+constexpr unsigned kPanelWaitLimit = 1u << 22;
+__device__ __forceinline__ bool panel_gave_up(const int* status) {
+  return *reinterpret_cast<const volatile int*>(status + SW_TIMEOUT) != 0;
+}
+// Messages to a CTA whose wait ran out may still be in flight when all have been sent (after the last
+// cluster barrier), and its shared memory has to outlive them: remote stores take about a microsecond,
+// this a millisecond.
+__device__ __forceinline__ void drain_messages() {
+  for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+}
+
 __device__ __forceinline__ uint32_t mapa_u32(uint32_t saddr, uint32_t rank) {
   uint32_t r;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
@@ -328,7 +344,7 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) panel_reg_kernel(PanelArg
           if (alive) {
             unsigned it = 0;
             while (!tc::mbar_try_wait(&bar[par], (uint32_t)(jj >> 1) & 1u))
-              if (++it >= (1u << 22)) {
+              if (++it >= kPanelWaitLimit) {
                 atomicExch(a.status + SW_TIMEOUT, 2);
                 alive = false;
                 break;
@@ -356,7 +372,7 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) panel_reg_kernel(PanelArg
         }
         if (mine) *pcol = l;
         s_ipiv[jj] = p;  // every thread the same value
-        if (G > 1 && tid == 0 && jj + 2 < ncols) tc::mbar_expect_tx(&bar[par], G * kMsgBytes);
+        if (G > 1 && tid == 0 && alive && jj + 2 < ncols) tc::mbar_expect_tx(&bar[par], G * kMsgBytes);
       }
       if (tid < kRegPanelRows) s_pos[tid] = pos;
     }
@@ -416,6 +432,11 @@ __global__ void __launch_bounds__(kRegPanelThreads, 1) panel_reg_kernel(PanelArg
   if (G > 1) {
     cluster_arrive();
     cluster_wait();
+    if (panel_gave_up(a.status)) {
+      if (b == 0) no_interchanges(a.sw, a.ipiv, a.k0, ncols, tid, NT);
+      if (!alive) drain_messages();
+      return;
+    }
   }
   // write back: row lr to its position
   for (int rg = 0; rg < FW; ++rg) {
@@ -552,6 +573,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) panel_sub_kernel(SubArgs<T> a)
     if (b == 0 && a.c0 == 0) *a.sw.n_extra = 0;
   }
   if (tid < W) s_prow[tid] = -1;
+  if (b == 0 && tid < wc) a.prow[a.c0 + tid] = a.c0 + tid;  // a row for panel_rest_kernel should none become the pivot
   for (int c = 0; c < wc; ++c) {
     const T* src = a.W + (size_t)(a.k0 + r0) + (size_t)(a.k0 + a.c0 + c) * a.ld;
     for (int lr = tid; lr < nloc; lr += NT) cp_async_elem(P + (size_t)c * rpcp + lr, src + lr);
@@ -656,7 +678,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) panel_sub_kernel(SubArgs<T> a)
           if (alive) {
             unsigned it = 0;
             while (!tc::mbar_try_wait(&bar[par], (uint32_t)(jl >> 1) & 1u))
-              if (++it >= (1u << 22)) {
+              if (++it >= kPanelWaitLimit) {
                 atomicExch(a.status + SW_TIMEOUT, 3);
                 alive = false;
                 break;
@@ -687,7 +709,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) panel_sub_kernel(SubArgs<T> a)
           if (held[q]) pcol[q * NT] = l[q];
         }
         s_ipiv[jl] = p;  // every thread the same value
-        if (tid == 0 && jl + 2 < wc) tc::mbar_expect_tx(&bar[par], G * kMsgBytes);
+        if (tid == 0 && alive && jl + 2 < wc) tc::mbar_expect_tx(&bar[par], G * kMsgBytes);
       }
     }
     __syncthreads();
@@ -738,6 +760,9 @@ __global__ void __launch_bounds__(kSubThreads, 1) panel_sub_kernel(SubArgs<T> a)
   }
   cluster_arrive();
   cluster_wait();
+  // (before the last sub-panel positions are only compared and prow is the one index)
+  const bool last = a.c0 + W >= a.ncols, gave_up = last && panel_gave_up(a.status);
+  if (gave_up && b == 0) no_interchanges(a.sw, a.ipiv, a.k0, a.ncols, tid, NT);
   // the sub-panel back in place, positions, pivots
 #pragma unroll
   for (int q = 0; q < RPT; ++q) {
@@ -749,8 +774,8 @@ __global__ void __launch_bounds__(kSubThreads, 1) panel_sub_kernel(SubArgs<T> a)
       for (int c = 0; c < W; ++c)
         if (c < wc) dst[(size_t)c * a.ld] = P[(size_t)c * rpcp + lr];
     }
-    a.pos[r0 + lr] = pos[q];
-    if (a.c0 + W >= a.ncols) {  // last sub-panel: the step's row interchanges
+    a.pos[r0 + lr] = gave_up ? r0 + lr : pos[q];
+    if (last && !gave_up) {  // the step's row interchanges
       const int src = a.k0 + r0 + lr, dst = a.k0 + pos[q];
       if (pos[q] < a.ncols) {
         a.sw.top_src[pos[q]] = src;
@@ -762,7 +787,8 @@ __global__ void __launch_bounds__(kSubThreads, 1) panel_sub_kernel(SubArgs<T> a)
     }
   }
   if (tid < wc && s_prow[tid] >= 0) a.prow[a.c0 + tid] = r0 + s_prow[tid];
-  if (b == 0 && tid < wc) a.ipiv[a.k0 + a.c0 + tid] = a.k0 + s_ipiv[tid];
+  if (b == 0 && tid < wc && !gave_up) a.ipiv[a.k0 + a.c0 + tid] = a.k0 + s_ipiv[tid];
+  if (!alive) drain_messages();
 }
 
 // 64 rows per CTA of 256 threads: 2 x 32 rows, four column groups.
