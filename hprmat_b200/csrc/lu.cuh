@@ -248,7 +248,10 @@ __global__ void __launch_bounds__(NT, 1) panel_kernel(PanelArgs<T> a) {
     long long* tr = a.trace ? a.trace + (size_t)j * kPanelTraceW : nullptr;
     if (tr && b == 0 && tid == 0) tr[0] = device_ns();
     // every CTA has posted its candidate of column j
-    if (!grid_wait(a.status + SW_BARRIER, a.status + SW_TIMEOUT, (unsigned)a.G * (j + 1), 1)) return;
+    if (!grid_wait(a.status + SW_BARRIER, a.status + SW_TIMEOUT, (unsigned)a.G * (j + 1), 1)) {
+      if (b == 0) no_interchanges(a.sw, a.ipiv, a.k0, ncols, tid, NT);
+      return;
+    }
     if (tr && b == 0 && tid == 0) tr[2] = device_ns();
     // the winning key names the pivot row; its owner CTA is row / rpc
     if (tid == 0) {

@@ -1,6 +1,6 @@
 // One panel of the LU on the emulator: <kernel> <f|d> <N> <k0> <ncols> <CTAs> <drop_src> <drop_dst> <drop_from>
 // <wait limit> <status word before> <output file>.  kernel: reg, tall (its sub-panels, updates and placing) or
-// grid.  Writes the sizes, the status words, pivots and interchange lists, the number of guard bytes that
+// grid (absent: its last CTA never runs).  Writes the sizes, the status words, pivots and interchange lists, the number of guard bytes that
 // were written and of the emulator's faults, then the matrix before and after and the LU planes.
 #include "emulate.h"
 #include "panel.cuh"
@@ -82,7 +82,7 @@ int run(char** v) {
     if (kind == "reg")
       emu::launch(G, kRegPanelThreads, true, [&] { panel_reg_kernel<T, kNB>(a); });
     else
-      emu::launch(G, 256, true, [&] { panel_kernel<T, kNB, 256>(a); });
+      emu::launch(kind == "absent" ? G - 1 : G, 256, true, [&] { panel_kernel<T, kNB, 256>(a); });
   }
   const size_t hits = W.hits() + cand.hits() + rowj.hits() + ubuf.hits() + xrows.hits() + lists.hits() + ipiv.hits() +
                       status.hits() + pos.hits() + prow.hits() + keys.hits() + lup.hits();

@@ -132,3 +132,13 @@ def test_a_panel_that_gives_up(emulator, tmp_path, kernel, n, k0, ncols, ctas, p
     else:  # the sub-panels factor their own rows in place
         assert np.array_equal(np.delete(q.after, slice(k0, k0 + ncols), 1), np.delete(q.before, slice(k0, k0 + ncols), 1))
         assert np.array_equal(q.after[:k0], q.before[:k0])
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+def test_a_grid_panel_that_gives_up(emulator, tmp_path, prec):
+    """The panel over the whole grid, one CTA missing at its barrier (300 polls): no interchanges, nothing
+    written."""
+    q = Panel(emulator, tmp_path, "absent", prec, 100, 32, 32, 3, limit=300)
+    assert (q.timeout, q.outside, q.faults, q.n_extra) == (1, 0, 0, 0)
+    assert list(q.top) == list(q.ipiv[32:64]) == list(range(32, 64))
+    assert np.array_equal(q.after, q.before) and not q.planes.any()
