@@ -634,10 +634,6 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   st.nb = NB;
   st.nsteps = nsteps;
   int* status = c->status.as<int>();
-  if (c->side) {  // a factorisation that ended in an error may have left its panel there
-    HPR_CUDA_TRY(cudaEventRecord(c->side_ev[2], c->side));
-    HPR_CUDA_TRY(cudaStreamWaitEvent(c->stream, c->side_ev[2], 0));
-  }
   HPR_CUDA_TRY(cudaMemsetAsync(status, 0, SW_COUNT * sizeof(int), c->stream));
   const int G0 = std::min(c->nsm, std::max(1, (N + 31) / 32));
   TRY(c->stage.ensure((size_t)2 * G0 * NB * sizeof(T) + (size_t)NB * sizeof(unsigned long long) +
@@ -1160,13 +1156,18 @@ static int factor(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, int nb, 
   NvtxRange nv(mixed ? "hprmat.factor.mixed" : "hprmat.factor.fp64");
   if (N >= PivotKey<T>::kMaxRows)
     return fail(HPRMAT_B200_ERR_UNSUPPORTED, "order %d beyond the pivot keys' row range", N);
+  int s = HPRMAT_B200_OK;
   switch (nb) {
-    case 128: return factor_impl<T, 128>(c, W, ld, N, mixed, st);
-    case 64: return factor_impl<T, 64>(c, W, ld, N, mixed, st);
-    case 32: return factor_impl<T, 32>(c, W, ld, N, mixed, st);
-    case 16: return factor_impl<T, 16>(c, W, ld, N, mixed, st);
+    case 128: s = factor_impl<T, 128>(c, W, ld, N, mixed, st); break;
+    case 64: s = factor_impl<T, 64>(c, W, ld, N, mixed, st); break;
+    case 32: s = factor_impl<T, 32>(c, W, ld, N, mixed, st); break;
+    case 16: s = factor_impl<T, 16>(c, W, ld, N, mixed, st); break;
+    default: return fail(HPRMAT_B200_ERR_UNSUPPORTED, "unsupported block size %d", nb);
   }
-  return fail(HPRMAT_B200_ERR_UNSUPPORTED, "unsupported block size %d", nb);
+  // An error may leave a look-ahead panel on its own stream, and the caller's next writes to W are
+  // ordered behind the context's stream alone.
+  if (s != HPRMAT_B200_OK && c->side) cudaStreamSynchronize(c->side);
+  return s;
 }
 
 // Forward and backward substitution with the stored factors, in place on X (N x nrhs).

@@ -107,7 +107,29 @@ def last_solve_of_an_interval(rt):
     assert e.value.status == rt.nat.ERR_TIMEOUT and str(WAIT_SITE) in str(e.value)
 
 
-SCENARIOS = {f.__name__: f for f in (last_solve_of_a_dense_call, last_solve_of_an_interval)}
+def error_beside_a_panel(rt):
+    """The look-ahead's panel is on its own stream when a launch beside it fails: the call does not return
+    while that panel may still write into the matrix."""
+    for prec, n in (("mixed", 700), ("fp64", 700)):
+        state = {}
+
+        def on_launch(name, op):
+            if state.get("panel") and op.stream != state["panel"]:
+                state["failed"] = True
+                return 1
+            if op.completion_event:  # the panel beside which the update runs
+                state["panel"] = op.stream
+        ctx = rt.api.Context(precision=prec)
+        rt.tune(ctx, b"lookahead", 512)
+        rt.on_launch = on_launch
+        with pytest.raises(rt.nat.HprmatError) as e:
+            ctx.solve_linear(np.eye(n), np.ones((n, 1)))
+        assert state.get("failed") and e.value.status == rt.nat.ERR_CUDA
+        mine = [o for o in rt.ops if o[2] == state["panel"]]
+        assert mine[-1][0] == "sync", mine[-1]
+
+
+SCENARIOS = {f.__name__: f for f in (last_solve_of_a_dense_call, last_solve_of_an_interval, error_beside_a_panel)}
 
 
 @pytest.fixture(scope="module")
