@@ -51,6 +51,7 @@ void hprmat::set_last_error(cudaError_t e, const char* what, const char* file, i
   char buf[512];
   snprintf(buf, sizeof(buf), "%s: %s (%s:%d)", cudaGetErrorString(e), what, file, line);
   g_last_error = buf;
+  cudaGetLastError();  // reported now: the next launch check on this thread must not find it again
 }
 void hprmat::set_last_error_msg(const char* msg) { g_last_error = msg; }
 
@@ -967,9 +968,11 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
         cfg.attrs = at;
         cfg.numAttrs = ahead ? 2 : 1;
         const cudaError_t e = cudaLaunchKernelEx(&cfg, pkc, pa);
-        if (e != cudaSuccess)
+        if (e != cudaSuccess) {
+          cudaGetLastError();
           return fail(HPRMAT_B200_ERR_CUDA, "cluster panel launch (step %d, %d CTAs of %d rows, %zu B shared): %s", s,
                       Gc, rpcc, smc, cudaGetErrorString(e));
+        }
         ++c->launches;
         if (ahead) TRY(ahead_update());
         TRY(ahead_join());
@@ -3059,9 +3062,11 @@ static int hess_reduce_blocked(hprmat_b200_ctx* c, double2* A, long ld, int N, d
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 2;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, hb_col_cluster_kernel, ca);
-    if (e != cudaSuccess)
+    if (e != cudaSuccess) {
+      cudaGetLastError();
       return fail(HPRMAT_B200_ERR_CUDA, "Hessenberg column step (%d CTAs of %d rows): %s", Gc, rpc,
                   cudaGetErrorString(e));
+    }
     ++c->launches;
     return HPRMAT_B200_OK;
   };

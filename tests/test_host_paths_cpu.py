@@ -129,7 +129,26 @@ def error_beside_a_panel(rt):
         assert mine[-1][0] == "sync", mine[-1]
 
 
-SCENARIOS = {f.__name__: f for f in (last_solve_of_a_dense_call, last_solve_of_an_interval, error_beside_a_panel)}
+def a_launch_error_is_reported_once(rt):
+    """The runtime also keeps a failed launch's error for cudaGetLastError; the next call on the thread must not
+    find it there."""
+    def solve(prec):
+        ctx = rt.api.Context(precision=prec)
+        rt.on_launch = rt.norms([1.0, 1e-14])
+        ctx.solve_linear(np.eye(300), np.ones((300, 1)))
+    for prec, kernel in (("mixed", "panel_reg_kernel"), ("fp64", "zgemm_dmma_kernel"), ("mixed", "full_inverse_kernel")):
+        failed = []
+        rt.on_launch = lambda name, op: failed.append(name) or 1 if kernel in name and not failed else 0
+        ctx = rt.api.Context(precision=prec)
+        with pytest.raises(rt.nat.HprmatError) as e:
+            ctx.solve_linear(np.eye(300), np.ones((300, 1)))
+        assert failed and e.value.status == rt.nat.ERR_CUDA
+        solve("mixed")
+        solve("fp64")
+
+
+SCENARIOS = {f.__name__: f for f in (last_solve_of_a_dense_call, last_solve_of_an_interval, error_beside_a_panel,
+                                   a_launch_error_is_reported_once)}
 
 
 @pytest.fixture(scope="module")
