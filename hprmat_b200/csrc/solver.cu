@@ -171,8 +171,9 @@ struct hprmat_b200_ctx {
   int panel_rpc_min = 32;    // fewest panel rows per CTA
   double growth_limit = 1e6;  // mixed path: pivot growth above which C(E) is factorised in FP64
   bool panel_cluster = true;  // panels that fit in one 16-CTA cluster use panel_reg_kernel
-  signed char cluster_ok[2][17] = {};  // per element size (float2, double2) and cluster size:
-                                       // 0 unknown, 1 schedulable, -1 not
+  // per panel_reg_kernel instance (float2, double2; block size 16, 32, 64, 128) and cluster size:
+  // 0 unknown, 1 schedulable (and large clusters allowed for that kernel), -1 not
+  signed char cluster_ok[2][4][17] = {};
   int gmres_m = 12;          // longest FGMRES cycle per outer step (<= kGmresMaxM)
   double inner_tol0 = 1e-7;  // first cycle stops once the residual fell this much
   bool zero_start = false;   // refinement starts from X = 0 instead of the FP32 solution
@@ -867,7 +868,7 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
   auto pk = panel_kernel<T, NB, NT>;
   auto pkc = panel_reg_kernel<T, NB>;
   auto cluster_fits = [&](int g) -> bool {  // can the GPU hold a cluster of g such CTAs
-    signed char& ok = c->cluster_ok[sizeof(T) == sizeof(double2)][g];
+    signed char& ok = c->cluster_ok[sizeof(T) == sizeof(double2)][NB == 16 ? 0 : NB == 32 ? 1 : NB == 64 ? 2 : 3][g];
     if (ok == 0) {
       const size_t sm = panel_reg_smem<T, NB>(rpc_max_c);
       ok = -1;

@@ -1,5 +1,7 @@
 """The cluster panel of the LU (panel.cuh): dense solves at the edges of its row split, sub-panels
 and cluster sizes, against numpy's solution."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -107,3 +109,17 @@ def test_fp64_lookahead(n):
             x = ctx.solve_linear(a, b)
             assert np.abs(a @ x - b).max() <= 8 * n * 2.0 ** -53 * np.abs(a).sum(1).max() * np.abs(x).max()
             assert np.array_equal(xs.setdefault(rows, x), x)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_block_sizes_in_one_context(precision):
+    """One context at several block sizes in turn, on clusters of 16 CTAs each: the bound of the first test."""
+    n = 600
+    a = _matrix(n, False)
+    b = np.random.default_rng(n).uniform(-1, 1, (n, 2)) + 0j
+    with api.Context(precision=precision, max_refine=8, tol=1e-15) as ctx:
+        for nb in (64, 32, 16, 64) if precision == "fp64" else (128, 64, 32, 16, 128):
+            ctx.opts.panel_nb = nb
+            nat.check(nat.load().hprmat_b200_set_opts(ctx._h, ctypes.byref(ctx.opts)))
+            x = ctx.solve_linear(a, b, allow_unconverged=True)
+            assert np.abs(a @ x - b).max() <= 8 * n * 2.0 ** -53 * np.abs(a).sum(1).max() * np.abs(x).max()

@@ -147,8 +147,23 @@ def a_launch_error_is_reported_once(rt):
         solve("fp64")
 
 
+def block_sizes_in_turn(rt):
+    """One context that factorises at one block size and then at another: each is a panel kernel of its own,
+    and launches on clusters of more than 8 CTAs."""
+    for prec in ("mixed", "fp64"):
+        sizes = (128, 64, 32, 16) if prec == "mixed" else (64, 32, 16)
+        ctx = rt.api.Context(precision=prec)
+        for nb in sizes + sizes[::-1]:
+            ctx.opts.panel_nb = nb
+            rt.nat.check(rt.nat.load().hprmat_b200_set_opts(ctx._h, ctypes.byref(ctx.opts)))
+            rt.on_launch = rt.norms([1.0, 1e-14])
+            del rt.ops[:]
+            ctx.solve_linear(np.eye(600), np.ones((600, 1)))
+            assert max(o[4] for o in rt.ops if "panel_reg_kernel" in o[1]) == 16
+
+
 SCENARIOS = {f.__name__: f for f in (last_solve_of_a_dense_call, last_solve_of_an_interval, error_beside_a_panel,
-                                   a_launch_error_is_reported_once)}
+                                   a_launch_error_is_reported_once, block_sizes_in_turn)}
 
 
 @pytest.fixture(scope="module")
