@@ -2825,6 +2825,7 @@ static int scan_workers_ready(hprmat_b200_ctx* c, int nworkers, int nr, double r
     w->panel_rpc_min = c->panel_rpc_min;
     w->gmres_m = c->gmres_m;
     w->tcplan.max_grid = c->tcplan.max_grid;
+    w->lookahead = c->lookahead;
     w->reuse_max_inner = c->reuse_max_inner;
     w->lu_held = false;
     TRY(hprmat_b200_rmat_ini(w, nr, 1, rmax, zrma.data()));

@@ -162,8 +162,22 @@ def block_sizes_in_turn(rt):
             assert max(o[4] for o in rt.ops if "panel_reg_kernel" in o[1]) == 16
 
 
+def scan_workers_take_the_look_ahead(rt):
+    """`lookahead` 0 on a context holds for the workers of its scans: no panel beside an update, no stream for
+    it."""
+    for rows in (512 * 4, 0):
+        w = rt.workloads.production(nch=12, nr=60, rmax=20.0, energy=5.0)
+        ctx = rt.api.Context(precision="fp64")
+        rt.tune(ctx, b"lookahead", rows)
+        beside = []
+        rt.on_launch = lambda name, op: beside.append(name) if op.completion_event else 0
+        ctx.rmatrix_scan([(w.lval, w.cpot, np.array([w.qk] * 2), np.array([w.eta] * 2))], 20.0, 60, nworkers=2)
+        assert bool(beside) == (rows > 0)
+
+
 SCENARIOS = {f.__name__: f for f in (last_solve_of_a_dense_call, last_solve_of_an_interval, error_beside_a_panel,
-                                   a_launch_error_is_reported_once, block_sizes_in_turn)}
+                                   a_launch_error_is_reported_once, block_sizes_in_turn,
+                                   scan_workers_take_the_look_ahead)}
 
 
 @pytest.fixture(scope="module")
