@@ -76,8 +76,9 @@ int hprmat_b200_dev_counters(hprmat_b200_ctx* ctx, unsigned long long* launches,
                       take 16 where the GPU holds such a cluster;
      "lookahead"      LU: fewest rows of a trailing matrix that is updated beside the next panel
                       (default 2048, a quarter of it for FP64; 0: never);
-     "hess_workers"   shifted scan: J-pi blocks in flight at once, each on a worker context
-                      of its own, 1..8 (3). */
+     "hess_workers"   shifted scan: most J-pi blocks in flight at once, each on a worker context
+                      of its own, 1..8 (3); the scan takes the fewest workers whose largest share of
+                      the work is within 10 % of what it is on that many. */
 int hprmat_b200_dev_set_tuning(hprmat_b200_ctx* ctx, const char* key, int value);
 
 /* Failure-path check: one CTA waits, with a limit of `spins` polls (4096 .. 2^24), on a device

@@ -235,6 +235,24 @@ def test_shifted_scan_workers_give_identical_results():
     ctx.close()
 
 
+def test_shifted_scan_on_three_workers():
+    """Three blocks of one order, which hess_workers 3 puts in flight together (two workers serve the blocks of
+    the test above, one of which is most of the work): U, nopen and status bitwise as on one worker."""
+    from hprmat_b200 import _native as nat
+    args = []
+    for seed in (510, 511, 512):
+        w = workloads.production(seed=seed, nch=14, nr=60, rmax=20.0, energy=1.0)
+        ks = [workloads.channel_kinematics(e, w.thresholds, w.hm, w.params.z1z2) for e in (5.0, 12.0, 21.0)]
+        args.append((w.lval, w.cpot, np.array([k[0] for k in ks]), np.array([k[1] for k in ks])))
+    with api.Context(precision="mixed") as ctx:
+        out = []
+        for nw in (1, 3):
+            nat.check(nat.load().hprmat_b200_dev_set_tuning(ctx._h, b"hess_workers", nw))
+            out.append(ctx.rmatrix_scan(args, 20.0, 60, method="shifted"))
+    for one, three in zip(*out):
+        assert all(np.array_equal(x, y) for x, y in zip(one, three))
+
+
 def test_shifted_scan_on_a_config3_sample():
     """A sample of the energy-scan configuration (blocks of 4..64 channels x 60 points, energies
     in 1-30 MeV): the shifted scan against the oracle on every fourth energy of three blocks,

@@ -175,9 +175,26 @@ def scan_workers_take_the_look_ahead(rt):
         assert bool(beside) == (rows > 0)
 
 
+def workers_of_the_shifted_scan(rt):
+    """`hess_workers` bounds the blocks in flight: three blocks of one order take three workers of 3, one of
+    1; blocks of 4, 13 and 24 channels, the largest of which is most of the work, take two."""
+    def workers(channels, limit):
+        blocks = []
+        for nch in channels:
+            w = rt.workloads.production(nch=nch, nr=60, rmax=20.0, energy=5.0)
+            blocks.append((w.lval, w.cpot, np.array([w.qk]), np.array([w.eta])))
+        ctx = rt.api.Context(precision="mixed")
+        rt.tune(ctx, b"hess_workers", limit)
+        del rt.ops[:]
+        ctx.rmatrix_scan(blocks, 20.0, 60, method="shifted", raise_on_unit_error=False)
+        return len({o[2] for o in rt.ops if "hb_gemv_kernel" in o[1]})
+    assert [workers((9, 9, 9), n) for n in (1, 2, 3)] == [1, 2, 3]
+    assert workers((4, 13, 24), 3) == 2
+
+
 SCENARIOS = {f.__name__: f for f in (last_solve_of_a_dense_call, last_solve_of_an_interval, error_beside_a_panel,
                                    a_launch_error_is_reported_once, block_sizes_in_turn,
-                                   scan_workers_take_the_look_ahead)}
+                                   scan_workers_take_the_look_ahead, workers_of_the_shifted_scan)}
 
 
 @pytest.fixture(scope="module")
