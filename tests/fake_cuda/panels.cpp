@@ -1,5 +1,6 @@
 // One panel of the LU on the emulator: <kernel> <f|d> <N> <k0> <ncols> <CTAs> <drop_src> <drop_dst> <drop_from>
-// <wait limit> <status word before> <output file>.  kernel: reg, tall (its sub-panels, updates and placing) or
+// <wait limit> <status word before> <odd value> <output file>.  odd value: 1 a NaN in the panel, 2 an infinity, 3 a
+// column of NaN, 4 nothing but NaN, 5 a row of infinities.  kernel: reg, tall (its sub-panels, updates and placing) or
 // grid (absent: its last CTA never runs).  Writes the sizes, the status words, pivots and interchange lists, the number of guard bytes that
 // were written and of the emulator's faults, then the matrix before and after and the LU planes.
 #include "emulate.h"
@@ -27,6 +28,13 @@ int run(char** v) {
     W.p[i].x = rnd();
     W.p[i].y = rnd();
   }
+  const int odd = atoi(v[12]);
+  for (int c = k0; c < k0 + ncols; ++c)
+    for (int r = k0; r < N; ++r) {
+      auto& e = W.p[r + (size_t)c * ld];
+      if ((odd <= 2 && odd > 0 && r == k0 + 7 && c == k0 + 3) || (odd == 3 && c == k0 + 5) || odd == 4 || (odd == 5 && r == k0 + 9))
+        e.y = odd == 2 || odd == 5 ? INFINITY : NAN;
+    }
   const std::vector<T> before(W.p, W.p + W.n);
   status.p[SW_TIMEOUT] = atoi(v[11]);
   for (int i = 0; i < 3 * kNB + 1; ++i) lists.p[i] = -(1 << 18);  // what an unwritten list may hold
@@ -86,7 +94,7 @@ int run(char** v) {
   }
   const size_t hits = W.hits() + cand.hits() + rowj.hits() + ubuf.hits() + xrows.hits() + lists.hits() + ipiv.hits() +
                       status.hits() + pos.hits() + prow.hits() + keys.hits() + lup.hits();
-  FILE* f = fopen(v[12], "wb");
+  FILE* f = fopen(v[13], "wb");
   const int head[4] = {ld, SW_TIMEOUT, (int)std::min<size_t>(hits, 1u << 30), emu::faults.load()};
   fwrite(head, sizeof(int), 4, f);
   fwrite(status.p, sizeof(int), SW_COUNT, f);
@@ -99,6 +107,6 @@ int run(char** v) {
 }
 
 int main(int argc, char** argv) {
-  if (argc != 13) return 2;
+  if (argc != 14) return 2;
   return argv[2][0] == 'd' ? run<double2>(argv) : run<float2>(argv);
 }

@@ -123,3 +123,26 @@ def test_block_sizes_in_one_context(precision):
             nat.check(nat.load().hprmat_b200_set_opts(ctx._h, ctypes.byref(ctx.opts)))
             x = ctx.solve_linear(a, b, allow_unconverged=True)
             assert np.abs(a @ x - b).max() <= 8 * n * 2.0 ** -53 * np.abs(a).sum(1).max() * np.abs(x).max()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, complex(0.0, -np.inf)])
+@pytest.mark.parametrize("n", [100, 400, 1500, 3333])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_nan_and_infinity(precision, n, value):
+    """One entry that is not finite, in the first panel, in U12 or in the last rows: the call ends, with an error
+    or a solution (for a NaN one that is not finite; an infinite pivot has a finite limit), and the context solves
+    the next system to the first test's bound."""
+    a = _matrix(n, False)
+    b = np.random.default_rng(n).uniform(-1, 1, (n, 1)) + 0j
+    with api.Context(precision=precision, max_refine=8, tol=1e-15) as ctx:
+        for i, j in ((n // 2, 3), (5, n - 2), (n - 1, n - 1)):
+            bad = a.copy()
+            bad[i, j] = value
+            try:
+                x = ctx.solve_linear(bad, b, allow_unconverged=True)
+            except api.HprmatError as e:
+                assert e.status in (nat.SINGULAR, nat.PIVOT_GROWTH)
+            else:
+                assert not (np.isnan(value) and np.isfinite(x).all())
+        x = ctx.solve_linear(a, b, allow_unconverged=True)
+    assert np.abs(a @ x - b).max() <= 8 * n * 2.0 ** -53 * np.abs(a).sum(1).max() * np.abs(x).max()

@@ -54,9 +54,9 @@ def emulator(tmp_path_factory):
 
 
 class Panel:
-    def __init__(self, exe, tmp, kernel, prec, n, k0, ncols, ctas, drop=(-1, -1, 0), limit=1 << 30, flag=0):
+    def __init__(self, exe, tmp, kernel, prec, n, k0, ncols, ctas, drop=(-1, -1, 0), limit=1 << 30, flag=0, odd=0):
         f = str(tmp / "out.bin")
-        subprocess.run([exe, kernel, prec, *map(str, (n, k0, ncols, ctas, *drop, limit, flag)), f], check=True, timeout=300)
+        subprocess.run([exe, kernel, prec, *map(str, (n, k0, ncols, ctas, *drop, limit, flag, odd)), f], check=True, timeout=300)
         raw = open(f, "rb").read()
         real, cplx = (np.float64, np.complex128) if prec == "d" else (np.float32, np.complex64)
         ld, sw, self.outside, self.faults = np.frombuffer(raw, np.int32, 4)
@@ -142,3 +142,20 @@ def test_a_grid_panel_that_gives_up(emulator, tmp_path, prec):
     assert (q.timeout, q.outside, q.faults, q.n_extra) == (1, 0, 0, 0)
     assert list(q.top) == list(q.ipiv[32:64]) == list(range(32, 64))
     assert np.array_equal(q.after, q.before) and not q.planes.any()
+
+
+@pytest.mark.parametrize("odd", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("kernel,n,k0,ncols,ctas", [("reg", 40, 8, 32, 1), ("reg", 100, 32, 32, 3), ("tall", 150, 32, 32, 16)])
+@pytest.mark.parametrize("prec", ["f", "d"])
+def test_panels_of_nan_and_infinity(emulator, tmp_path, kernel, n, k0, ncols, ctas, prec, odd):
+    """A NaN, an infinity, a column or a whole panel of NaN, a row of infinities: the rows' order stays a
+    permutation, no store leaves the buffers, and the panel is not finite where it was not before."""
+    q = Panel(emulator, tmp_path, kernel, prec, n, k0, ncols, ctas, odd=odd)
+    assert (q.outside, q.faults, q.timeout) == (0, 0, 0)
+    order = np.arange(n)
+    order[k0:k0 + ncols] = q.top[:ncols]
+    order[q.dst[:q.n_extra]] = q.src[:q.n_extra]
+    assert sorted(order) == list(range(n))
+    assert all(k0 + j <= p < n for j, p in enumerate(q.ipiv[k0:k0 + ncols]))
+    assert not np.isfinite(q.after[k0:, k0:k0 + ncols]).all()
+    assert np.array_equal(np.delete(q.after, slice(k0, k0 + ncols), 1), np.delete(q.before, slice(k0, k0 + ncols), 1))
