@@ -306,6 +306,11 @@ inline void st_async16(uint32_t dst, uint4 v, uint32_t bar) {
   memcpy(emu::resolve(dst), &v, 16);
   emu::mbar_step((emu::Mbar*)emu::resolve(bar), 0, -16);
 }
+inline void st_cluster_u32(uint32_t dst, unsigned v) {
+  std::lock_guard<std::mutex> lk(emu::mu);
+  if (emu::cta->cluster->left[dst >> 27]) return emu::fault("remote store into a CTA that has left");
+  memcpy(emu::resolve(dst), &v, 4);
+}
 namespace tc {
 inline uint32_t smem_u32(const void* p) { return emu::address(p); }
 inline void mbar_init(uint64_t* b, uint32_t n) {

@@ -13,7 +13,8 @@ CSRC = os.path.join(ROOT, "hprmat_b200", "csrc")
 NB = 32
 # inline assembly, restated in emulate.h
 RESTATED = ["cp_async_elem", "cp_async_wait_all", "device_ns", "grid_arrive", "grid_wait", "smem_u32", "mbar_init",
-            "mbar_try_wait", "mbar_expect_tx", "cluster_arrive", "cluster_wait", "mapa_u32", "st_async16"]
+            "mbar_try_wait", "mbar_expect_tx", "cluster_arrive", "cluster_wait", "mapa_u32", "st_async16",
+            "st_cluster_u32"]
 
 
 def _without(src, name):
