@@ -82,7 +82,11 @@ typedef struct {
   int nb;                   /* LU block size used */
   int n;                    /* order of the solved system */
   int nrhs;
-  double rel_residual;      /* final ||B - C X||_F / ||B||_F, evaluated in FP64 */
+  double rel_residual;      /* last ||B - C X||_F / ||B||_F formed, evaluated in FP64.  Mixed R-matrix calls
+                               that meet tol after a refinement step apply one more LU solve to that residual
+                               (it takes the error in R further down) and form none after it: this
+                               and the histories then describe X before that solve, which the
+                               counts above leave out too */
   double surface_change;    /* relative change of R in the last refinement step (-1: n/a) */
   double residual_floor;    /* estimated rounding floor of the relative FP64 residual (0: n/a) */
   double floor_history[9];  /* the floor estimate at each outer step */
