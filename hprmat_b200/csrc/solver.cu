@@ -892,10 +892,12 @@ static int factor_impl(hprmat_b200_ctx* c, T* W, long ld, int N, bool mixed, LUS
     }
     return ok == 1;
   };
-  const int sub_rows = 16 * kSubThreads * (sizeof(T) == sizeof(double2) ? 2 : 4);
+  // Most rows per CTA of a sub-panel: as many as a thread takes (panel_sub_kernel's RPT), and as the shared
+  // memory holds beside the static arrays, which is fewer: 1687 (FP64 843), a panel of 26992 (13488) rows.
+  int sub_rpc = kSubThreads * (sizeof(T) == sizeof(double2) ? 2 : 4);
+  while (sub_rpc > 0 && panel_sub_smem<T>(sub_rpc) + 16 * 1024 > (size_t)c->smem_optin) --sub_rpc;
   auto tall_fits = [&](int m) -> bool {  // sub-panels on one 16-CTA cluster
-    return NB >= 2 * kSubW && m <= sub_rows && panel_sub_smem<T>((m + 15) / 16) + 16 * 1024 <= (size_t)c->smem_optin &&
-           cluster_fits(16);
+    return NB >= 2 * kSubW && m <= 16 * sub_rpc && cluster_fits(16);
   };
   const int ahead_min = mixed ? c->lookahead : c->lookahead / 4;
   if ((mixed || pair) && c->panel_cluster && ahead_min > 0 && N - NB >= ahead_min && c->nsm > 32 && cluster_fits(16)) {
