@@ -455,9 +455,9 @@ static int pick_nb(const hprmat_b200_ctx* c, int N, size_t elem, int preferred) 
 static int wave_prepare(hprmat_b200_ctx* c, const LUState& st) {
   const int N = st.N, ns = st.nsteps;
   c->wave_ready = false;
-  // super blocks of 4 blocks (2 for nsteps < 4): a quarter of the dependency links, at the
-  // price of 4x larger diagonal inverses in the one-time preparation
-  const int sb = c->wave_sb > 0 ? c->wave_sb : (ns >= 4 ? 4 : 2);
+  // super blocks of 4 blocks: a quarter of the dependency links, at the price of 4x larger
+  // diagonal inverses in the one-time preparation (orders of few blocks come here only with wave_sb set)
+  const int sb = c->wave_sb > 0 ? c->wave_sb : 4;
   const long sig_ld = (N + 3) / 4 * 4;
   TRY(c->wsig.ensure((size_t)ns * sig_ld * sizeof(int)));
   TRY(c->wperm.ensure((size_t)3 * N * sizeof(int) + 64));
