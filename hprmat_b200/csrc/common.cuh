@@ -162,41 +162,10 @@ enum StatusWord {
   SW_COUNT = 8
 };
 
-// Bounded grid-wide barrier for cooperative launches.  `target` = number of CTAs times
-// the barrier's ordinal (1-based) since the counter was zeroed.  Thread 0 arrives with a
-// release-ordered add (publishing the CTA's earlier writes, ordered by __syncthreads) and
-// polls with acquire loads; the error flag is looked at only every 4096 polls.  Returns
-// false when the wait exceeded its limit; the caller must then stop touching shared data
-// and return.
-__device__ inline bool grid_barrier(int* counter, int* timeout_flag, unsigned target, int site) {
-  __syncthreads();
-  __shared__ int s_ok;
-  if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
-    int ok = 1;
-    for (unsigned spins = 1;; ++spins) {
-      unsigned v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-      if (v >= target) break;
-      if ((spins & 4095u) == 0) {
-        int tf;
-        asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(tf) : "l"(timeout_flag) : "memory");
-        if (tf != 0) { ok = 0; break; }
-        if (spins >= (1u << 26)) {  // seconds: something is wrong
-          atomicExch(timeout_flag, site);
-          ok = 0;
-          break;
-        }
-      }
-    }
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-// The two halves of grid_barrier, so that a CTA can work between arriving and waiting.
-// grid_arrive is called by thread 0 after a __syncthreads that orders the CTA's writes.
+// Bounded grid-wide barrier for cooperative launches, in two halves so that a CTA can work between
+// arriving and waiting: `target` = number of CTAs times the barrier's ordinal (1-based) since the counter
+// was zeroed.  Arrivals are release-ordered adds (they publish the CTA's earlier writes), the wait polls with
+// acquire loads.  grid_arrive is called by thread 0 after a __syncthreads that orders the CTA's writes.
 __device__ inline void grid_arrive(int* counter) {
   asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
 }
