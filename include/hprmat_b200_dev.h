@@ -106,7 +106,8 @@ long long hprmat_b200_dev_factorizations(hprmat_b200_ctx* ctx, int reset);
 int hprmat_b200_dev_mesh(int nr, int ns, double rmax, double* tc, double* blo, double* q2, double* q1,
                          double* zrma);
 
-/* Tracing of the wavefront triangular solves of the mixed path.  With enable != 0 every
+/* Tracing of the wavefront triangular solves of the mixed path (more than 10 blocks, or "wave_sb" set:
+   smaller orders solve with explicit inverses and record nothing).  With enable != 0 every
    later sweep records, per unit (block row x right-hand-side group, in dependency order),
    four device-clock stamps in ns: the producer starts the unit, the last dependency flag
    was seen, the accumulator was complete, the block was published.
@@ -114,8 +115,8 @@ int hprmat_b200_dev_mesh(int nr, int ns, double rmax, double* tc, double* blo, d
    the last backward sweep (2 x units x 4 values, at most cap) and stores units. */
 int hprmat_b200_dev_wave_trace(hprmat_b200_ctx* ctx, int enable);
 int hprmat_b200_dev_wave_trace_read(hprmat_b200_ctx* ctx, long long* out, int cap, int* units);
-/* With tracing enabled, the panel factorisations of block steps 0 and nsteps/2 also record
-   per column `width` device-clock stamps: CTA 0 at column start, candidate posted, grid
+/* With tracing enabled, the panel factorisations of block steps 0 and nsteps/2 that run over the
+   whole grid (panel_cluster 0, or more rows than the cluster kernels take) also record per column `width` device-clock stamps: CTA 0 at column start, candidate posted, grid
    barrier passed, pivot row in place, update done, then each CTA's barrier arrival.
    Copies 2 x 128 x width values (at most cap). */
 int hprmat_b200_dev_panel_trace_read(hprmat_b200_ctx* ctx, long long* out, int cap, int* width);
