@@ -116,9 +116,10 @@ int hprmat_b200_dev_mesh(int nr, int ns, double rmax, double* tc, double* blo, d
 int hprmat_b200_dev_wave_trace(hprmat_b200_ctx* ctx, int enable);
 int hprmat_b200_dev_wave_trace_read(hprmat_b200_ctx* ctx, long long* out, int cap, int* units);
 /* With tracing enabled, the panel factorisations of block steps 0 and nsteps/2 that run over the
-   whole grid (panel_cluster 0, or more rows than the cluster kernels take) also record per column `width` device-clock stamps: CTA 0 at column start, candidate posted, grid
-   barrier passed, pivot row in place, update done, then each CTA's barrier arrival.
-   Copies 2 x 128 x width values (at most cap). */
+   whole grid (panel_cluster 0, or more rows than the cluster kernels take) also record per column
+   `width` device-clock stamps: CTA 0 at column start, candidate posted, grid barrier passed, pivot
+   row in place, update done, then each CTA's barrier arrival.  Copies 2 x 128 x width values (at
+   most cap). */
 int hprmat_b200_dev_panel_trace_read(hprmat_b200_ctx* ctx, long long* out, int cap, int* width);
 
 #ifdef __cplusplus
