@@ -4,7 +4,8 @@
 //
 // Storage: the matrix W is column-major with leading dimension ld (complex elements).
 // Block step s factors columns [k0, k0+ncols) with k0 = s*nb:
-//   1. the panel: panel_reg_kernel (panel.cuh) where the rows fit in one thread-block cluster,
+//   1. the panel: panel_reg_kernel (panel.cuh) where the rows fit in one thread-block cluster, its
+//      sub-panels (panel_sub_kernel, panel_rest_kernel) where 16 columns of them do,
 //      else panel_kernel -- cooperative launch, the panel rows spread over all SMs and held
 //                           in shared memory; one grid barrier per column: every CTA posts
 //                           its local |re|+|im| maximum (the modulus LAPACK's izamax uses)
@@ -69,8 +70,8 @@ __device__ __forceinline__ void no_interchanges(const StepSwaps& sw, int* ipiv, 
   if (tid == 0) *sw.n_extra = 0;
 }
 
-// End of a panel factorisation: the CTA's factored rows back into W, its L21 rows into the LU planes (mixed path), and from CTA 0 the pivots, the growth
-// and the step's row-interchange list.
+// End of panel_kernel: the CTA's factored rows back into W, its L21 rows into the LU planes (mixed
+// path), and from CTA 0 the pivots, the growth and the step's row-interchange list.
 template <typename T, int NB, int NT>
 __device__ void panel_finish(const PanelArgs<T>& a, const T* P, int rpcp, int r0, int nloc, const int* s_loc_ipiv,
                              unsigned s_growth, int b, int tid) {
